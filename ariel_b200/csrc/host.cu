@@ -252,7 +252,9 @@ long long layout_bytes(const Layout& L) {
         add(nc, 8);
         add(nc, 4);
     }
-    add(3 * std::max(1ll, L.maxch), 8);
+    add(6 * std::max(1ll, L.maxch), 8);
+    add(k, 16);      // resident solve: scene table
+    add(32 * k, 4);  // and arrival counters
     add(L.nbricks, 16);  // brick list
     add(k + 1, 4);       // brick bases
     add(L.nbricks, 4);   // brick flags
@@ -650,7 +652,10 @@ ariel_status build_state(ariel_sim* s, std::vector<HostParticles>& hp, const ari
         ARIEL_TRY(dalloc(s, &A.d32, nc));
     }
     A.max_chunks = std::max(1ll, maxch);
-    ARIEL_TRY(dalloc(s, &A.partial, 3 * A.max_chunks));
+    ARIEL_TRY(dalloc(s, &A.partial, 6 * A.max_chunks));
+    ARIEL_TRY(dalloc(s, &A.res, k));
+    ARIEL_TRY(dalloc(s, &A.res_count, 32 * (size_t)k));
+    A.flscan = s->flscan;
     // bricks of the ordered sweeps: every scene's brick grid, listed by level I+J+K, then scene
     // and position (the order the sweeps take them in)
     sweep_brick(s->prm, A.bx, A.by, A.bz);
@@ -706,6 +711,16 @@ ariel_status build_state(ariel_sim* s, std::vector<HostParticles>& hp, const ari
     A.S = S;
     s->pcg_blocks = pcg_max_blocks(s->device, s->mode, s->prm.pcg_blocks_per_sm);
     if (s->prm.pcg_grid_blocks > 0) s->pcg_blocks = std::min(s->pcg_blocks, (int)s->prm.pcg_grid_blocks);
+    A.res_blocks = pcg_res_blocks(s->device, s->mode);
+    if (s->prm.pcg_grid_blocks > 0) A.res_blocks = std::min(A.res_blocks, (int)s->prm.pcg_grid_blocks);
+    A.all_resident = A.all_small = 1;
+    for (int i = 0; i < k; ++i) {
+        const long long n = s->descs[i].dim;
+        if (chunk_bound(n * n * n) > res_chunk_limit(A.res_blocks, s->mode) ||
+            !res_fits(s->mode, 2 * chunk_size(n * n * n)))
+            A.all_resident = 0;
+        if (chunk_size(n * n * n) > 2 * kPcgThreads) A.all_small = 0;
+    }
     cudaStream_t st = s->stream;
     // scene table and prefixes
     ARIEL_CUDA(cudaMemcpyAsync(s->d_scenes, s->sh.data(), sizeof(SceneDev) * k, cudaMemcpyHostToDevice, st));

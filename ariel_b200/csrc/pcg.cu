@@ -21,6 +21,8 @@
 // and all blocks return.
 #include <cooperative_groups.h>
 
+#include <type_traits>
+
 #include "pcg.cuh"
 
 namespace ariel {
@@ -165,6 +167,16 @@ struct VT<kFp64> {
 // ------------------------------------------------------------------------------------------
 // Preparation: per-cell operator data, order-free preconditioner, FLUID predicate.
 // ------------------------------------------------------------------------------------------
+// The FLUID list follows the cells brick by brick (8 x 8 x 32 cells, cut off at the far walls)
+// instead of the whole grid's (i, j, k) order: a chunk of consecutive entries is then a compact
+// piece of the liquid, with about 0.6 neighbours outside it per cell where a chunk of whole grid
+// rows has 2.1, and still runs of up to 32 consecutive cells along z.
+__device__ __forceinline__ int list_order(int n, int i, int j, int k) {
+    const int i0 = i & ~7, j0 = j & ~7, k0 = k & ~31;
+    const int bi = min(8, n - i0), bj = min(8, n - j0), bk = min(32, n - k0);
+    return (i0 * n + j0 * bi) * n + k0 * bi * bj + ((i - i0) * bj + (j - j0)) * bk + (k - k0);
+}
+
 __global__ void k_prep_cells(PcgArgs A, uint32_t* pred) {
     const DevState& S = A.S;
     __shared__ long long pref_s[kMaxScenes + 1];
@@ -175,7 +187,9 @@ __global__ void k_prep_cells(PcgArgs A, uint32_t* pred) {
     const SceneDev& D = S.scenes[s];
     const int n = D.n;
     const uint8_t flag = S.flags[c];
-    pred[c] = flag == ARIEL_FLUID;
+    int i, j, k;
+    cell_ijk(D, c - D.c_begin, i, j, k);
+    pred[D.c_begin + list_order(n, i, j, k)] = flag == ARIEL_FLUID;
     if (flag != ARIEL_FLUID) {
         S.P[c] = 0.0f;
         if (S.P64) S.P64[c] = 0.0;
@@ -185,8 +199,6 @@ __global__ void k_prep_cells(PcgArgs A, uint32_t* pred) {
         A.pc32[c] = 0.0f;
         return;
     }
-    int i, j, k;
-    cell_ijk(D, c - D.c_begin, i, j, k);
     const int q[6][3] = {{i - 1, j, k}, {i + 1, j, k}, {i, j - 1, k}, {i, j + 1, k}, {i, j, k - 1}, {i, j, k + 1}};
     const float Lc = S.L[c];
     float d32 = 6.0f;
@@ -239,11 +251,17 @@ __global__ void k_prep_cells(PcgArgs A, uint32_t* pred) {
 // FLUID list, plus one 16-byte record per entry holding everything the solve needs about the
 // cell besides its vectors: index, neighbour mask and ADiag (fp32 bits for the fp32 modes, fp64
 // bits otherwise), so that a single load starts a cell's update.
-__global__ void k_fl_write(PcgArgs A, const uint32_t* pred, const uint32_t* scan) {
+__global__ void k_fl_write(PcgArgs A, const uint32_t* scan) {
+    const DevState& S = A.S;
+    __shared__ long long pref_s[kMaxScenes + 1];
+    load_prefix<kMaxScenes>(pref_s, S.c_pref, S.k);
     long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= A.S.nc) return;
-    if (!pred[c]) return;
-    const uint32_t t = scan[c];
+    if (c >= S.nc) return;
+    if (S.flags[c] != ARIEL_FLUID) return;
+    const SceneDev& D = S.scenes[find_scene(pref_s, S.k, c)];
+    int i, j, k;
+    cell_ijk(D, c - D.c_begin, i, j, k);
+    const uint32_t t = scan[D.c_begin + list_order(D.n, i, j, k)];
     const_cast<uint32_t*>(A.fl)[t] = (uint32_t)c;
     uint4 r;
     r.x = (uint32_t)c;
@@ -259,29 +277,72 @@ __global__ void k_fl_write(PcgArgs A, const uint32_t* pred, const uint32_t* scan
     A.rec[t] = r;
 }
 
-__global__ void k_pcg_tables(PcgArgs A, const uint32_t* scan) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// Per-scene tables of the solve, one block.  A scene of at most `limit` chunks is resident: it
+// gets a range of block positions inside one group of A.res_blocks (first fit by falling size,
+// so that small scenes fill the groups of the large ones).  The others keep their chunks in
+// ch_pref for the streaming kernel.
+constexpr int kTableThreads = 256;
+__global__ void __launch_bounds__(kTableThreads) k_pcg_tables(PcgArgs A, const uint32_t* scan, int limit) {
     const int k = A.S.k;
+    __shared__ int nch_s[kMaxScenes], order_s[kResMaxScenes], fill_s[kResMaxScenes];
     long long* flp = const_cast<long long*>(A.fl_pref);
     long long* chp = const_cast<long long*>(A.ch_pref);
-    long long acc = 0;
-    int any_ordered = 0;
-    for (int s = 0; s <= k; ++s) flp[s] = scan[A.S.c_pref[s]];
-    for (int s = 0; s < k; ++s) {
-        chp[s] = acc;
-        long long nf = flp[s + 1] - flp[s];
+    int ordered = 0;
+    for (int s = threadIdx.x; s <= k; s += kTableThreads) {
+        const long long b = scan[A.S.c_pref[s]];
+        flp[s] = b;
+        if (s == k) break;
+        const long long nf = scan[A.S.c_pref[s + 1]] - b;
         const int cs = chunk_size(nf);
-        acc += (nf + cs - 1) / cs;
+        nch_s[s] = (int)((nf + cs - 1) / cs);
         PcgScene& P = A.sc[s];
         P.nf = (int)nf;
         P.csize = cs;
         P.ordered = nf > 0 && (A.precond == ARIEL_PRECOND_MIC0 || P.ones > 0);
-        any_ordered |= P.ordered;
+        ordered |= P.ordered;
+    }
+    const int any_ordered = __syncthreads_or(ordered);
+    const bool may = limit > 0 && !any_ordered && k <= kResMaxScenes;
+    auto cpb_of = [&](int s) { return nch_s[s] > A.res_blocks ? 2 : 1; };  // chunks per block
+    auto resident = [&](int s) {
+        return may && nch_s[s] <= limit && res_fits(A.mode, cpb_of(s) * A.sc[s].csize);
+    };
+    if (may) {
+        for (int s = threadIdx.x; s < k; s += kTableThreads) {
+            int rank = 0;
+            for (int t = 0; t < k; ++t) rank += nch_s[t] > nch_s[s] || (nch_s[t] == nch_s[s] && t < s);
+            order_s[rank] = s;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    long long acc = 0;
+    int nstream = 0, partials = 0, groups = 0;
+    for (int s = 0; s < k; ++s) {
+        chp[s] = acc;
+        if (resident(s)) continue;
+        acc += nch_s[s];
+        ++nstream;
+        if (A.res) A.res[s] = make_int4(-1, 0, 0, 0);
     }
     chp[k] = acc;
+    for (int i = 0; may && i < k; ++i) {
+        const int s = order_s[i], nch = nch_s[s], G = A.res_blocks;
+        if (!resident(s)) continue;
+        const int m = (nch + cpb_of(s) - 1) / cpb_of(s);
+        int g = 0;
+        while (g < groups && fill_s[g] + m > G) ++g;
+        if (g == groups) fill_s[groups++] = 0;
+        A.res[s] = make_int4(g * G + fill_s[g], m, nch, partials);
+        A.res_count[32 * s] = 0u;
+        fill_s[g] += m;
+        partials += nch;
+    }
     A.ctl->all_done = 0;
     A.ctl->all_inner_done = 0;
     A.ctl->any_ordered = any_ordered;
+    A.ctl->nvirt = groups * A.res_blocks;
+    A.ctl->nstream = nstream;
 }
 
 // Data written by other blocks is read only after a grid barrier (whose acquire makes ordinary
@@ -1287,10 +1348,11 @@ cudaError_t launch_pcg_prepare(const PcgArgs& A, uint32_t* pred, uint32_t* scan,
     cudaError_t e = launch_scan_u32(pred, scan, S.nc, scan_tmp, st);
     if (e != cudaSuccess) return e;
     if (S.nc > 0) {
-        k_fl_write<<<grid_for(S.nc), kBlock, 0, st>>>(A, pred, scan);
+        k_fl_write<<<grid_for(S.nc), kBlock, 0, st>>>(A, scan);
         count_launch();
     }
-    k_pcg_tables<<<1, 32, 0, st>>>(A, scan);
+    const int limit = A.fast && A.mode != kRef32 ? res_chunk_limit(A.res_blocks, A.mode) : 0;
+    k_pcg_tables<<<1, kTableThreads, 0, st>>>(A, scan, limit);
     count_launch();
     return cudaGetLastError();
 }
@@ -1317,6 +1379,7 @@ struct SceneLocal {
     double bb, rr, rho, alpha, beta, target, rr_out;
     float alpha32, beta32, rho32;
     int iters, outer, done, inner_done, converged, nf;
+    int resident;  // solved by k_pcg_res
 };
 
 // Asynchronous 16-byte global -> shared copies (L1 bypassed), completed per thread.
@@ -1493,7 +1556,7 @@ template <int MODE>
 __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_fast(PcgArgs A) {
     using T = typename VT<MODE>::T;
     using T4 = typename V4<T>::type;
-    if (A.ctl->any_ordered) return;  // the ordered preconditioner runs in k_pcg
+    if (A.ctl->any_ordered || A.ctl->nstream == 0) return;  // k_pcg or k_pcg_res solves
     const DevState& S = A.S;
     const int k = S.k;
     __shared__ long long fl_s[kFastMaxScenes + 1], ch_s[kFastMaxScenes + 1];
@@ -1521,15 +1584,16 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_fast(PcgArgs A) {
     for (int i = threadIdx.x; i < k; i += blockDim.x) {
         SceneLocal z{};
         z.nf = A.sc[i].nf;
+        z.done = z.inner_done = z.resident = MODE != kRef32 && A.res[i].x >= 0;
         L[i] = z;
         csz_s[i] = A.sc[i].csize;
     }
     __syncthreads();
     const long long nch = ch_s[k];
     const long long MC = A.max_chunks;
-    double* part0 = A.partial;
-    double* part1 = A.partial + MC;
-    double* part2 = A.partial + 2 * MC;
+    // Two sets of partial sums used in turn: a block past one barrier may write its sums for the
+    // next while a slower block still reads those of the last.
+    auto part = [&](unsigned e, int i) { return A.partial + ((e & 1u) * 3 + i) * MC; };
     const unsigned long long tmo = A.timeout_ns;
     unsigned epoch = 0;
     // Chunk sums are reduced per warp at once but combined across warps only every kDefer
@@ -1553,9 +1617,9 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_fast(PcgArgs A) {
             v2 = warp_sum(v2);
             if (lane == 0) {
                 const long long ch = blockIdx.x + (long long)(jpend0 + jj) * gridDim.x;
-                part0[ch] = v0;
-                part1[ch] = v1;
-                part2[ch] = v2;
+                part(epoch, 0)[ch] = v0;
+                part(epoch, 1)[ch] = v1;
+                part(epoch, 2)[ch] = v2;
             }
         }
         __syncthreads();
@@ -1631,7 +1695,9 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_fast(PcgArgs A) {
         for (int s = wid; s < k; s += blockDim.x / 32) {
             if (L[s].inner_done && L[s].done) continue;
             double v0, v1, v2;
-            scene_sum3(part0, part1, part2, nsum, ch_s[s], ch_s[s + 1], v0, v1, v2);
+            // the sums written before the barrier that made `epoch` what it is now
+            scene_sum3(part(epoch - 1, 0), part(epoch - 1, 1), part(epoch - 1, 2), nsum, ch_s[s], ch_s[s + 1], v0, v1,
+                       v2);
             if (lane == 0) {
                 if (f(s, L[s], v0, v1, v2)) atomicAdd(&s_active, 1);
             }
@@ -2132,6 +2198,7 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_fast(PcgArgs A) {
     if (blockIdx.x == 0) {
         for (int s = threadIdx.x; s < k; s += blockDim.x) {
             const SceneLocal& P = L[s];
+            if (P.resident) continue;
             PcgScene o = load_sc(A.sc + s);
             o.bb = P.bb;
             o.rr = P.rr;
@@ -2169,6 +2236,8 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_fast(PcgArgs A) {
     }
 }
 
+#include "pcg_resident.cuh"
+
 template <int MODE>
 static cudaError_t coop_launch(const PcgArgs& A, int nblocks, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
@@ -2203,17 +2272,42 @@ static cudaError_t coop_launch_fast(const PcgArgs& A, int nblocks, cudaStream_t 
     return e;
 }
 
-// With the reference preconditioner and few enough scenes the fast kernel solves and the
-// general kernel returns at once; with an ordered preconditioner it is the other way round
-// (the choice is made on the device, from the preparation's FLUID-cell scan).
+template <int MODE, int R>
+static cudaError_t coop_launch_res(const PcgArgs& A, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)A.res_blocks);
+    cfg.blockDim = dim3(kResThreads);
+    cfg.dynamicSmemBytes = kResSmem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, k_pcg_res<MODE, R>, A);
+    count_launch();
+    return e;
+}
+
+// With the reference preconditioner and few enough scenes the resident kernel solves the scenes
+// that fit it, the streaming fast kernel the others (not launched when none can be too large),
+// and the general kernel returns at once; with an ordered preconditioner it is the other way
+// round (the choice is made on the device, from the preparation's FLUID-cell scan).
 cudaError_t launch_pcg_solve(const PcgArgs& A, int nblocks, cudaStream_t st) {
     cudaError_t e = cudaSuccess;
     if (A.fast) {
-        switch (A.mode) {
-            case kRef32: e = coop_launch_fast<kRef32>(A, nblocks, st); break;
-            case kFp64: e = coop_launch_fast<kFp64>(A, nblocks, st); break;
-            default: e = coop_launch_fast<kMixed>(A, nblocks, st); break;
+        const int limit = res_chunk_limit(A.res_blocks, A.mode);
+        if (limit > 0) {
+            e = A.mode == kFp64 ? coop_launch_res<kFp64, 2>(A, st) : coop_launch_res<kMixed, 2>(A, st);
+            if (e == cudaSuccess && !A.all_small)
+                e = A.mode == kFp64 ? coop_launch_res<kFp64, kResRounds>(A, st)
+                                    : coop_launch_res<kMixed, kResRounds>(A, st);
+            if (e != cudaSuccess) return e;
         }
+        if (A.mode == kRef32)
+            e = coop_launch_fast<kRef32>(A, nblocks, st);
+        else if (!A.all_resident)
+            e = A.mode == kFp64 ? coop_launch_fast<kFp64>(A, nblocks, st) : coop_launch_fast<kMixed>(A, nblocks, st);
         if (e != cudaSuccess) return e;
         if (A.precond != ARIEL_PRECOND_MIC0 && !A.may_be_ordered) return e;
     }
@@ -2253,6 +2347,22 @@ int pcg_max_blocks(int device, int mode, int per_sm_cap) {
     // add arrivals to every grid barrier.
     int cap = per_sm_cap > 0 ? per_sm_cap : 2;
     return sms * (per < cap ? per : cap);
+}
+
+int pcg_res_blocks(int device, int mode) {
+    if (mode == kRef32) return 0;
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    auto fits = [](const void* f) {
+        int per = 0;
+        return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmem) == cudaSuccess &&
+               cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, kResThreads, kResSmem) == cudaSuccess && per > 0;
+    };
+    const bool ok = mode == kFp64
+                        ? fits((const void*)k_pcg_res<kFp64, 2>) && fits((const void*)k_pcg_res<kFp64, kResRounds>)
+                        : fits((const void*)k_pcg_res<kMixed, 2>) && fits((const void*)k_pcg_res<kMixed, kResRounds>);
+    if (!ok) cudaGetLastError();
+    return ok ? sms : 0;  // 0: no scene is resident
 }
 
 cudaError_t launch_barrier_selftest(Barrier* bar, int* err, unsigned long long timeout_ns, cudaStream_t st) {

@@ -42,14 +42,16 @@ struct PcgCtl {
     int all_done;
     int all_inner_done;
     int any_ordered;
-    int pad;
+    int nvirt;    // block positions of the resident solve (whole groups of gridDim.x)
+    int nstream;  // scenes left to the streaming kernel
+    int pad[3];
 };
 
 struct Barrier {
     unsigned count;
     unsigned gen;
     int error;
-    int pad;
+    unsigned beat;  // exchanges completed by the resident solve (its waits' sign of progress)
 };
 
 struct PcgArgs {
@@ -66,10 +68,18 @@ struct PcgArgs {
     double tau, sigma;
     unsigned long long timeout_ns;
     // FLUID list
-    const uint32_t* fl;        // packed FLUID cells, scene by scene, ascending
+    const uint32_t* fl;        // packed FLUID cells, scene by scene, in list_order
     uint4* rec;                // per FLUID-list entry: (cell, neighbour mask, diagonal bits)
     const long long* fl_pref;  // k+1
-    const long long* ch_pref;  // k+1 chunk begins
+    const long long* ch_pref;  // k+1 chunk begins (scenes of the resident solve have none)
+    const uint32_t* flscan;    // packed cell in list_order -> FLUID-list position
+    // resident solve: per scene (first block position, positions, chunks, first partial) or
+    // position -1 when it is not resident; one arrival counter per scene, 128 bytes apart
+    int4* res;
+    unsigned* res_count;
+    int res_blocks;            // its blocks (one per SM)
+    int all_resident;          // every scene fits the resident solve whatever its FLUID count
+    int all_small;             // and has the smallest chunks
     // per-cell operator data (dense over packed cells)
     uint8_t* mask;   // bit d set: neighbour d (-x,+x,-y,+y,-z,+z) is FLUID
     double* diag;    // ADiag (fp32 value for REF32, fp64 otherwise)
@@ -89,7 +99,7 @@ struct PcgArgs {
     void* vb;        // fast single-reduction PCG: packed (p, x)
     double* r64;     // MIXED outer residual
     float* d32;      // MIXED inner correction
-    double* partial; // 3 * max chunks (three dot products per reduction)
+    double* partial; // two sets of 3 * max chunks (three dot products per reduction)
     long long max_chunks;
     // ordered wavefront sweeps: bricks of every scene sorted by level I+J+K (then scene, I, J,
     // K), each scene's brick grid starting at brick_base[s], one progress flag per brick
@@ -108,8 +118,9 @@ struct PcgArgs {
 cudaError_t launch_pcg_prepare(const PcgArgs& A, uint32_t* pred, uint32_t* scan, void* scan_tmp, cudaStream_t st);
 // The cooperative persistent PCG kernel.
 cudaError_t launch_pcg_solve(const PcgArgs& A, int nblocks, cudaStream_t st);
-// Blocks of the persistent kernel that fit on the device at once.
+// Blocks of the persistent kernel that fit on the device at once; the resident solve's.
 int pcg_max_blocks(int device, int mode, int per_sm_cap);
+int pcg_res_blocks(int device, int mode);
 // Bounded-wait self test (one arrival missing).
 cudaError_t launch_barrier_selftest(Barrier* bar, int* err, unsigned long long timeout_ns, cudaStream_t st);
 
@@ -136,6 +147,23 @@ inline long long chunk_bound(long long cells) {
     const long long lo = (cells + kChunkMin - 1) / kChunkMin;
     const long long hi = (cells + kChunkMax - 1) / kChunkMax;
     return std::min(lo, std::max(kChunkTarget, hi));
+}
+// The resident solve: scenes of at most two chunks per block (one block per SM) whose cells fit
+// its shared memory together with slots for neighbours in other blocks, of which bricks of the
+// FLUID list's order have about 0.6 per cell.
+constexpr int kResMaxChunks = 320;
+constexpr int kResMaxScenes = 128;  // as the streaming fast kernel
+constexpr size_t kResSmem = 225 * 1024;  // all of an SM's but 2 KB for the static part
+inline int res_chunk_limit(int blocks, int mode) { return mode == kRef32 ? 0 : std::min(2 * blocks, kResMaxChunks); }
+// Slots for neighbours in other blocks beside a block's `cells` cells (positions fit 13 bits).
+__host__ __device__ constexpr int res_halo_slots(int mode, int cells) {
+    const long long tb = mode == kFp64 ? 8 : 4;
+    const long long left = ((long long)kResSmem - 64 - cells * (5 * tb + 16)) / (tb + 4);
+    const long long most = 8190 - cells;
+    return (int)(left < most ? left : most);
+}
+__host__ __device__ constexpr bool res_fits(int mode, int cells) {
+    return 4 * res_halo_slots(mode, cells) >= 3 * cells;
 }
 constexpr int kBrickMaxCells = 2048;
 constexpr int kBrickMaxExt = 2744;

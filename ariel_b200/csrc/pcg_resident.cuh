@@ -1,0 +1,502 @@
+// pcg_resident.cuh -- the pressure solve of scenes of at most two chunks per SM (included by
+// pcg.cu after its helpers; FP64 and MIXED with the elementwise preconditioner).
+//
+// k_pcg_fast keeps every scene of the launch in step: one grid barrier and one pass over all
+// partial sums per iteration, and every cell's state crosses L2 in every iteration.  A scene that
+// fits the SMs needs neither:
+//   - a block keeps its one or two chunks for the whole solve.  r, w, s stay in registers, p, x,
+//     u and the operator data in shared memory.  Only cells with a neighbour in another block
+//     write (r, w, s, pc) to L2, for those blocks to read.  Neighbours inside the block take the
+//     owner's u from shared memory, computed once per cell instead of once per neighbour;
+//   - a block waits only for the blocks of its own scene, on the scene's own arrival counter.
+// Scenes are packed into groups of at most gridDim.x block positions; a block takes its position
+// of each group in turn, so small scenes run side by side and large ones one after another, each
+// out of shared memory, instead of all of them streaming through L2.
+//
+// MIXED to 1e-5, ms per solve, k_pcg_fast before -> here: 32^3 0.54 -> 0.33, 64^3 1.11 -> 0.68,
+// 128^3 3.90 -> 2.24 (10.0 -> 5.8 us per iteration); FP64 77^3 1.76 -> 1.30.  What an iteration of
+// the 128^3 dam break spends, in SM cycles of about 11,000: 2,400 own update and halo, 2,500 the
+// operator (shared-memory bandwidth: 11 words per cell), 900 block sums, 2,500-3,500 arrival and
+// wait (a release, a reduction and an acquire through L2), 2,200 reading 291 partials and the fp64
+// divisions of alpha and beta.  At 64^3 the last three are 5,500 of 6,700 cycles.
+//
+// The arithmetic, the chunk of every cell, the entries of every thread and every summation tree
+// are those of k_pcg_fast, so both kernels give the same bits.
+#pragma once
+
+__device__ __forceinline__ float4 ldcg4(const float4* p) { return __ldcg(p); }
+__device__ __forceinline__ double4 ldcg4(const double4* p) {
+    const double2* q = reinterpret_cast<const double2*>(p);
+    const double2 a = __ldcg(q), b = __ldcg(q + 1);
+    return make_double4(a.x, a.y, b.x, b.y);
+}
+
+// One block per SM: two halves of kPcgThreads threads, each with a chunk.  Fewer arrivals and
+// pollers make the barrier cheaper than two blocks per SM do (148 against 291 blocks: 2.2 against
+// 2.9 us for an arrival, the wait and the reading of three sums per chunk).
+constexpr int kResThreads = 2 * kPcgThreads;
+constexpr int kResRounds = kChunkMax / kPcgThreads;
+constexpr unsigned kResOut = 0x1fff;  // a neighbour without a slot of u
+static_assert(2 * kChunkMax + 2 * kChunkMax / 2 < (int)kResOut, "positions of u must fit 13 bits");
+
+// One block's part in one scene's solve; R: rounds of one cell per thread (csize <= 256 R).  False
+// when a wait gave up.
+template <int MODE, int R>
+__device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
+    using T = typename VT<MODE>::T;
+    using T2 = typename V2<T>::type;
+    using T4 = typename V4<T>::type;
+    constexpr int kWarps = kPcgThreads / 32;
+    // halo entries of a thread loaded ahead of alpha and beta, in registers
+    constexpr int kAhead = R <= 2 ? 2 : (MODE == kFp64 ? 2 : 5);
+    const DevState& S = A.S;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int half = tid / kPcgThreads, htid = tid % kPcgThreads, hwid = htid >> 5;
+    extern __shared__ __align__(16) unsigned char dyn[];
+    __shared__ double dsum[2][3][kWarps], total[3];
+    __shared__ int s_nhalo;
+    // the scene's solver state, kept by thread 0; the others read alpha, beta and stop
+    __shared__ struct {
+        double bb, rr, rho, alpha, beta, target, rr_out;
+        int iters, outer, converged, stop;
+    } st;
+    const T* pcv = MODE == kFp64 ? (const T*)(const void*)A.pc64 : (const T*)(const void*)A.pc32;
+    T4* const Av0 = (T4*)A.va0;
+    T4* const Av1 = (T4*)A.va1;
+    const unsigned long long tmo = A.timeout_ns;
+    const SceneDev& D = S.scenes[sc];
+    const int4 pl = A.res[sc];
+    // this block's first chunk and its chunks (cpb for all blocks but perhaps the last)
+    const int nch = pl.z, cpb = nch > pl.y ? 2 : 1;
+    const int ch0 = (v - pl.x) * cpb, ch = ch0 + half;
+    const bool mine = half < cpb && ch < nch;
+    const int n = D.n;
+    const int nf = A.sc[sc].nf, csize = A.sc[sc].csize;
+    // list positions of the block: [t0, t0 + blen); of this half: [base, base + len) from t0
+    const long long t0 = A.fl_pref[sc] + (long long)ch0 * csize;
+    const int blen = min(cpb * csize, nf - ch0 * csize);
+    const int base = half * csize;
+    const int len = mine ? min(csize, nf - ch * csize) : 0;
+    // Shared memory: per cell (p, x), the diagonal, pc, u, the cell index and three words of
+    // neighbour positions in u (x, y, z pairs of 13 bits; bit 26 of the first: some neighbour
+    // lies in another block); u continues with the halo -- the neighbours in other blocks --
+    // and a slot that stays 0 for neighbours that are not FLUID; the halo's cells.
+    const int cells = cpb * csize, hcap = res_halo_slots(MODE, cells), zero = cells + hcap;
+    T2* const px = reinterpret_cast<T2*>(dyn);
+    T* const dgs = reinterpret_cast<T*>(px + cells);
+    T* const pcs = dgs + cells;
+    T* const ub = pcs + cells;
+    uint32_t* const cs = reinterpret_cast<uint32_t*>(ub + zero + 1);
+    uint32_t* const nw = cs + cells;
+    uint32_t* const hcell = nw + 3 * cells;
+    const unsigned arrivals = (unsigned)pl.y;
+    unsigned* const count = A.res_count + 32 * (size_t)sc;
+    unsigned epoch = 0;
+    // The scene's partial sums, in two sets used in turn: a block can be one exchange ahead
+    // of another block of its scene, never two.
+    auto partial = [&](unsigned e) {
+        return A.partial + (e & 1 ? 3 * (size_t)A.max_chunks : 0) + 3 * (size_t)pl.w;
+    };
+    // Publishes the `nsum` sums of this block's chunks and waits for the scene's other blocks
+    // (nsum 0: a barrier).  False when the wait gave up.
+    auto arrive_wait = [&](int nsum, double a, double b, double c) -> bool {
+        ++epoch;
+        if (nsum > 0) {
+            a = warp_sum(a);
+            b = warp_sum(b);
+            if (nsum > 2) c = warp_sum(c);
+            if (lane == 0) {
+                dsum[half][0][hwid] = a;
+                dsum[half][1][hwid] = b;
+                dsum[half][2][hwid] = c;
+            }
+        }
+        __syncthreads();
+        if (hwid < nsum) {
+            // block_sum2's second step: its tree over a warp whose lanes past the eight warp
+            // sums hold zeros
+            double x = lane < kWarps ? dsum[half][hwid][lane] : 0.0;
+            static_assert(kWarps == 8, "three steps sum the warps");
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+            if (lane == 0 && mine) partial(epoch)[hwid * nch + ch] = x;
+        }
+        __syncthreads();
+        bool ok = true;
+        if (tid == 0) {
+            // release: orders the block's writes (collected by the barrier above) before the
+            // arrival; acquire: the others' writes before what follows the barrier below
+            red_release_add(count, 1u);
+            const unsigned want = epoch * arrivals;
+            unsigned spin = 0, beat = 0;
+            unsigned long long t_start = 0;
+            while (ld_acquire_cnt(count) < want) {
+                if ((++spin & 255u) != 0) continue;
+                // Bounded: gives up when nothing has moved for the time limit.  The beat
+                // counts the exchanges of all scenes, since a block of this scene may still
+                // be busy with a scene of an earlier group.
+                if (*(volatile int*)&A.bar->error) {
+                    ok = false;
+                    break;
+                }
+                const unsigned long long now = gtimer();
+                const unsigned bt = *(volatile unsigned*)&A.bar->beat;
+                if (t_start == 0 || bt != beat) {
+                    t_start = now;
+                    beat = bt;
+                } else if (now - t_start > tmo) {
+                    atomicExch(&A.bar->error, 1);
+                    if (S.dev_error) atomicExch(S.dev_error, 1);
+                    ok = false;
+                    break;
+                }
+            }
+            if (ch0 == 0) atomicAdd(&A.bar->beat, 1u);
+        }
+        return __syncthreads_and(ok) != 0;
+    };
+    // The scene's sums into total[], then `f` by thread 0; ends with a block barrier.  `ahead`
+    // issues loads to overlap with it: after those of the partials, but before them where their
+    // registers and those of the partials together would spill.
+    auto sums = [&](int nsum, auto&& ahead, auto&& f) {
+        constexpr int kU = (kResMaxChunks + 31) / 32;
+        static_assert(kU <= 16, "scene_sum3 takes these partials in one go");
+        if (R > 2) ahead();
+        double x[kU];
+        if (wid < nsum) {
+            const double* const p0 = partial(epoch) + wid * nch;
+#pragma unroll
+            for (int u = 0; u < kU; ++u) {
+                const int c0 = u * 32 + lane;
+                x[u] = c0 < nch ? __ldcg(p0 + c0) : 0.0;
+            }
+        }
+        if (R <= 2) ahead();
+        if (wid < nsum) {
+            double y = 0.0;
+#pragma unroll
+            for (int u = 0; u < kU; ++u) y += x[u];
+            y = warp_sum(y);
+            if (lane == 0) total[wid] = y;
+        }
+        if (wid < 3) asm volatile("bar.sync 1, 96;" ::: "memory");
+        if (tid == 0) f();
+        __syncthreads();
+    };
+
+    // ---- the block's operator data --------------------------------------------------------
+    if (tid == 0) {
+        st = {};
+        s_nhalo = 0;
+        ub[zero] = (T)0;
+    }
+    __syncthreads();
+    for (int o = base + htid; o < base + len; o += kPcgThreads) {
+        const uint4 rc = A.rec[t0 + o];
+        const uint32_t c = rc.x, m = rc.y;
+        T dg;
+        dec_diag(rc, dg);
+        int i, j, kk;
+        cell_ijk(D, (long long)c - D.c_begin, i, j, kk);
+        bool out = false;
+        auto code = [&](int d, int a, int b, int e) -> uint32_t {
+            if (!((m >> d) & 1u)) return (uint32_t)zero;
+            const long long p = (long long)A.flscan[D.c_begin + list_order(n, a, b, e)] - t0;
+            if (p >= 0 && p < blen) return (uint32_t)p;
+            out = true;
+            // one slot for each active lane, in lane order
+            const unsigned act = __activemask();
+            const int lead = __ffs(act) - 1;
+            int h = 0;
+            if (lane == lead) h = atomicAdd(&s_nhalo, __popc(act));
+            h = __shfl_sync(act, h, lead) + __popc(act & ((1u << lane) - 1u));
+            if (h >= hcap) return kResOut;
+            hcell[h] = c + (uint32_t)nb_off(d, n);
+            return (uint32_t)(cells + h);
+        };
+        const uint32_t x0 = code(0, i - 1, j, kk), x1 = code(1, i + 1, j, kk);
+        const uint32_t y0 = code(2, i, j - 1, kk), y1 = code(3, i, j + 1, kk);
+        const uint32_t z0 = code(4, i, j, kk - 1), z1 = code(5, i, j, kk + 1);
+        cs[o] = c;
+        dgs[o] = dg;
+        pcs[o] = pcv[c];
+        nw[o] = x0 | x1 << 13 | (out ? 1u << 26 : 0u);
+        nw[cells + o] = y0 | y1 << 13;
+        nw[2 * cells + o] = z0 | z1 << 13;
+    }
+    // (every thread reads back only its own entries of cs, dgs, pcs, nw and px)
+    __syncthreads();
+    const bool over = s_nhalo > hcap;  // some neighbours have no slot: read where needed
+    const int nhalo = min(s_nhalo, hcap);
+
+    const T scale = (T)(1.0 / (double)D.ax_h);
+    const int cap = A.max_iters > 0 ? A.max_iters : n * n * n;
+    T r[R], w[R], sv[R];
+
+    for (int outer = 0;; ++outer) {
+        // ---- residual r = b - A x, |b|^2 ------------------------------------------------
+        double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+        for (int o = base + htid; o < base + len; o += kPcgThreads) {
+            const long long c = cs[o];
+            const double bv = (double)S.D[c];
+            const double xc = __ldcg(S.P64 + c);
+            const double ax = ax_diag<double>(A, D, c, xc, [&](long long q) { return __ldcg(S.P64 + q); });
+            const double rv = bv - ax;
+            if (MODE == kMixed)
+                A.r64[c] = rv;
+            else
+                ((T*)A.r)[c] = (T)rv;
+            a0 += rv * rv;
+            a1 += bv * bv;
+        }
+        if (!arrive_wait(2, a0, a1, 0.0)) return false;
+        sums(2, [] {}, [&] {
+            const double rr = total[0];
+            if (outer == 0) st.bb = total[1];
+            st.rr_out = rr;
+            if (MODE == kMixed) st.outer += 1;
+            const double lim2 = A.tol * A.tol * st.bb;
+            const double abs_eps = (double)(1.0e-2f * (float)(n * n * n));
+            bool conv = false;
+            if (A.stop_rule == ARIEL_STOP_REL)
+                conv = rr <= lim2;
+            else if (MODE == kMixed)
+                conv = outer > 0 && rr <= abs_eps;
+            if (conv) {
+                st.stop = 1;
+                st.converged = 1;
+            } else if (MODE == kMixed && (st.outer > A.max_outer || st.iters >= cap)) {
+                st.stop = 1;
+            }
+            if (st.stop) return;
+            st.rr = rr;
+            if (MODE == kMixed) {
+                // the correction solve stops at the final tolerance itself (its fp32
+                // residual); the true residual then decides whether another sweep is needed
+                const double a = A.inner_tol * A.inner_tol * rr;
+                const double b = A.stop_rule == ARIEL_STOP_REL ? lim2 : 0.0;
+                st.target = a > b ? a : b;
+            } else {
+                st.target = A.stop_rule == ARIEL_STOP_REL ? lim2 : abs_eps;
+            }
+        });
+        if (st.stop) break;
+        // ---- u = M r, w = A u, p = 0 ----------------------------------------------------
+        auto r0 = [&](long long q) -> T {
+            return MODE == kMixed ? (T)__ldcg(A.r64 + q) : __ldcg((const T*)A.r + q);
+        };
+        a0 = a1 = 0.0;
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+            const int o = base + htid + q * kPcgThreads;
+            if (o < base + len) {
+                const long long c = cs[o];
+                const uint32_t m = A.mask[c];
+                const T rv = r0(c), pcc = pcs[o];
+                const T uv = (rv * pcc) * pcc;
+                T acc = dgs[o] * uv;
+#pragma unroll
+                for (int d = 0; d < 6; ++d)
+                    if (m & (1u << d)) {
+                        const long long qq = c + nb_off(d, n);
+                        const T pq = pcv[qq];
+                        acc -= (r0(qq) * pq) * pq;
+                    }
+                const T wv = acc * scale;
+                const T xv = MODE == kMixed ? (T)0 : (T)S.P64[c];
+                if (nw[o] >> 26) st4(Av0 + c, mk4<T>(rv, wv, (T)0, pcc));
+                r[q] = rv;
+                w[q] = wv;
+                sv[q] = (T)0;
+                px[o] = mk2<T>((T)0, xv);
+                a0 += (double)rv * (double)uv;
+                a1 += (double)wv * (double)uv;
+            }
+        }
+        if (!arrive_wait(2, a0, a1, 0.0)) return false;
+        // ---- iterations: k_pcg_fast's update of (r, w, s, p, x, u), one exchange each ---
+        // The halo comes from L2 as its owners' (r, w, s, pc) of the last iteration; the loads
+        // are issued as soon as the wait ends, ahead of alpha and beta.
+        for (int it = 0;; ++it) {
+            const T4* const Ac = (it & 1) ? Av1 : Av0;
+            T4* const An = (it & 1) ? Av0 : Av1;
+            T4 eh[kAhead];
+            auto load_halo = [&] {
+#pragma unroll
+                for (int u = 0; u < kAhead; ++u) {
+                    const int h = tid + u * kResThreads;
+                    if (h < nhalo) eh[u] = ldcg4(Ac + hcell[h]);
+                }
+            };
+            if (it == 0)
+                sums(2, load_halo, [&] {
+                    st.rho = total[0];
+                    st.alpha = total[1] != 0.0 ? total[0] / total[1] : 0.0;
+                    st.beta = 0.0;
+                    st.stop = 0;
+                });
+            else
+                sums(3, load_halo, [&] {
+                    const double g = total[0], d = total[1];
+                    st.iters += 1;
+                    st.rr = total[2];
+                    const bool conv = total[2] <= st.target;
+                    if (conv || st.iters >= cap) {
+                        if (MODE != kMixed) st.converged = conv;
+                        st.stop = 1;
+                        return;
+                    }
+                    const double beta = st.rho != 0.0 ? g / st.rho : 0.0;
+                    const double den = d - (st.alpha != 0.0 ? beta * g / st.alpha : 0.0);
+                    st.beta = beta;
+                    st.alpha = den != 0.0 ? g / den : 0.0;
+                    st.rho = g;
+                });
+            if (st.stop) break;
+            const T al = (T)st.alpha, bt = (T)st.beta;
+            auto u_of = [&](const T4& e) -> T {
+                const T sq = e.y + bt * e.z;
+                const T rq = e.x - al * sq;
+                return (rq * e.w) * e.w;
+            };
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                const int h = tid + u * kResThreads;
+                if (h < nhalo) ub[cells + h] = u_of(eh[u]);
+            }
+            for (int h = tid + kAhead * kResThreads; h < nhalo; h += kResThreads)
+                ub[cells + h] = u_of(ldcg4(Ac + hcell[h]));
+#pragma unroll
+            for (int q = 0; q < R; ++q) {
+                const int o = base + htid + q * kPcgThreads;
+                if (o < base + len) {
+                    const T pc = pcs[o];
+                    const T2 b = px[o];
+                    const T s1 = w[q] + bt * sv[q];
+                    const T ui = (r[q] * pc) * pc;
+                    const T pv = ui + bt * b.x;
+                    const T xv = b.y + al * pv;
+                    const T rn = r[q] - al * s1;
+                    sv[q] = s1;
+                    r[q] = rn;
+                    px[o] = mk2<T>(pv, xv);
+                    ub[o] = (rn * pc) * pc;
+                }
+            }
+            __syncthreads();
+            a0 = a1 = a2 = 0.0;
+            auto apply = [&](auto has_out) {
+#pragma unroll
+                for (int q = 0; q < R; ++q) {
+                    const int o = base + htid + q * kPcgThreads;
+                    if (o < base + len) {
+                        const uint32_t nb[3] = {nw[o], nw[cells + o], nw[2 * cells + o]};
+                        const T un = ub[o];
+                        T a = dgs[o] * un;
+#pragma unroll
+                        for (int d = 0; d < 6; ++d) {
+                            const unsigned p = (d & 1 ? nb[d / 2] >> 13 : nb[d / 2]) & 0x1fffu;
+                            if (decltype(has_out)::value && p == kResOut)
+                                a -= u_of(ldcg4(Ac + cs[o] + nb_off(d, n)));
+                            else
+                                a -= ub[p];  // 0 where the neighbour is not FLUID
+                        }
+                        const T wn = a * scale;
+                        w[q] = wn;
+                        if (nb[0] >> 26) st4(An + cs[o], mk4<T>(r[q], wn, sv[q], pcs[o]));
+                        if (MODE == kMixed) {
+                            // products of two floats are exact in double, so the fused sums
+                            // round as the separate ones
+                            const double dr = (double)r[q], du = (double)un;
+                            a0 = __fma_rn(dr, du, a0);
+                            a1 = __fma_rn((double)wn, du, a1);
+                            a2 = __fma_rn(dr, dr, a2);
+                        } else {
+                            a0 += (double)r[q] * (double)un;
+                            a1 += (double)wn * (double)un;
+                            a2 += (double)r[q] * (double)r[q];
+                        }
+                    }
+                }
+            };
+            if (over)
+                apply(std::true_type{});
+            else
+                apply(std::false_type{});
+            if (!arrive_wait(3, a0, a1, a2)) return false;
+        }
+        __syncthreads();
+        if (tid == 0) st.stop = 0;
+        // fold the solve's x back: MIXED adds the correction to x64, FP64 stores x64
+        for (int o = base + htid; o < base + len; o += kPcgThreads) {
+            const uint32_t c = cs[o];
+            S.P64[c] = MODE == kMixed ? S.P64[c] + (double)px[o].y : (double)px[o].y;
+        }
+        if (MODE != kMixed) break;
+        if (!arrive_wait(0, 0.0, 0.0, 0.0)) return false;
+    }
+    if (ch0 == 0 && tid == 0) {
+        PcgScene o = load_sc(A.sc + sc);
+        o.bb = st.bb;
+        o.rr = st.rr;
+        o.rho = st.rho;
+        o.alpha = st.alpha;
+        o.beta = st.beta;
+        o.rr_out = st.rr_out;
+        o.target = st.target;
+        o.iters = st.iters;
+        o.outer = st.outer;
+        o.done = 1;
+        o.inner_done = 1;
+        o.converged = st.converged;
+        A.sc[sc] = o;
+        PcgTotals& Tt = A.totals[sc];
+        const int sweeps = MODE == kMixed ? st.outer : 1;
+        Tt.solves += 1;
+        Tt.iterations += st.iters;
+        Tt.outer += sweeps;
+        Tt.cell_iterations += (double)nf * (double)st.iters;
+        Tt.cell_outer += (double)nf * (double)sweeps;
+        Tt.not_converged += st.converged ? 0 : 1;
+    }
+    for (int o = base + htid; o < base + len; o += kPcgThreads) {
+        const uint32_t c = cs[o];
+        S.P[c] = (float)S.P64[c];
+    }
+    return true;
+}
+
+// R = 2 takes the scenes of small chunks, without the code (and its registers) of rounds that none
+// of their threads has; R = kResRounds the others.
+template <int MODE, int R>
+__global__ void __launch_bounds__(kResThreads, 1) k_pcg_res(PcgArgs A) {
+    if (A.ctl->any_ordered) return;  // the ordered preconditioner runs in k_pcg
+    const DevState& S = A.S;
+    const int tid = threadIdx.x, nvirt = A.ctl->nvirt, k = S.k;
+    __shared__ int s_scene;
+    if (R == 2 && blockIdx.x == 0)
+        for (int s = tid; s < k; s += kResThreads) {
+            const int4 e = A.res[s];
+            if (e.x < 0 || e.z > 0) continue;
+            // a scene without FLUID cells: solved as it is
+            PcgScene o = load_sc(A.sc + s);
+            o.outer = MODE == kMixed ? 1 : 0;
+            o.done = o.inner_done = o.converged = 1;
+            A.sc[s] = o;
+            A.totals[s].solves += 1;
+            A.totals[s].outer += 1;
+        }
+    for (int v = blockIdx.x; v < nvirt; v += gridDim.x) {
+        __syncthreads();
+        if (tid == 0) s_scene = -1;
+        __syncthreads();
+        for (int s = tid; s < k; s += kResThreads) {
+            const int4 e = A.res[s];
+            if (v >= e.x && v < e.x + e.y && (A.sc[s].csize <= 2 * kPcgThreads) == (R == 2)) s_scene = s;
+        }
+        __syncthreads();
+        const int sc = s_scene;
+        if (sc < 0) continue;  // no chunk for this block in this group
+        if (!res_scene<MODE, R>(A, sc, v)) return;
+    }
+}
