@@ -713,13 +713,15 @@ ariel_status build_state(ariel_sim* s, std::vector<HostParticles>& hp, const ari
     if (s->prm.pcg_grid_blocks > 0) s->pcg_blocks = std::min(s->pcg_blocks, (int)s->prm.pcg_grid_blocks);
     A.res_blocks = pcg_res_blocks(s->device, s->mode);
     if (s->prm.pcg_grid_blocks > 0) A.res_blocks = std::min(A.res_blocks, (int)s->prm.pcg_grid_blocks);
-    A.all_resident = A.all_small = 1;
+    A.all_resident = A.res_blocks > 0;
+    A.classes = 0;
     for (int i = 0; i < k; ++i) {
+        // over every FLUID count that the scene's grid allows
         const long long n = s->descs[i].dim;
-        if (chunk_bound(n * n * n) > res_chunk_limit(A.res_blocks, s->mode) ||
-            !res_fits(s->mode, 2 * chunk_size(n * n * n)))
+        const int most = chunk_size(n * n * n);
+        for (int c = kChunkMin; c <= most; c += kChunkAlign) A.classes |= 1 << res_class(k, c);
+        if (chunk_bound(n * n * n) > std::min(kResMaxChunks, A.res_blocks * res_max_cpb(s->mode, k, most)))
             A.all_resident = 0;
-        if (chunk_size(n * n * n) > 2 * kPcgThreads) A.all_small = 0;
     }
     cudaStream_t st = s->stream;
     // scene table and prefixes

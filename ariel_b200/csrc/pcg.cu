@@ -277,17 +277,19 @@ __global__ void k_fl_write(PcgArgs A, const uint32_t* scan) {
     A.rec[t] = r;
 }
 
-// Per-scene tables of the solve, one block.  A scene of at most `limit` chunks is resident: it
-// gets a range of block positions inside one group of A.res_blocks (first fit by falling size,
-// so that small scenes fill the groups of the large ones).  The others keep their chunks in
-// ch_pref for the streaming kernel.
+// Per-scene tables of the solve, one block.  A resident scene gets a range of block positions
+// inside one group of A.res_blocks; the scenes of a class take as few chunks per block as put them
+// all in one group, and are packed into groups by falling size (first fit).  The others keep their
+// chunks in ch_pref for the streaming kernel.
 constexpr int kTableThreads = 256;
-__global__ void __launch_bounds__(kTableThreads) k_pcg_tables(PcgArgs A, const uint32_t* scan, int limit) {
-    const int k = A.S.k;
-    __shared__ int nch_s[kMaxScenes], order_s[kResMaxScenes], fill_s[kResMaxScenes];
+__global__ void __launch_bounds__(kTableThreads) k_pcg_tables(PcgArgs A, const uint32_t* scan) {
+    const int k = A.S.k, G = A.res_blocks;
+    __shared__ int nch_s[kMaxScenes], csz_s[kMaxScenes], order_s[kResMaxScenes], fill_s[kResMaxScenes];
+    __shared__ int need_s[kResClasses][4];  // positions of a class at 1, 2, 4, 8 chunks per block
     long long* flp = const_cast<long long*>(A.fl_pref);
     long long* chp = const_cast<long long*>(A.ch_pref);
     int ordered = 0;
+    for (int i = threadIdx.x; i < kResClasses * 4; i += kTableThreads) need_s[i / 4][i % 4] = 0;
     for (int s = threadIdx.x; s <= k; s += kTableThreads) {
         const long long b = scan[A.S.c_pref[s]];
         flp[s] = b;
@@ -295,6 +297,7 @@ __global__ void __launch_bounds__(kTableThreads) k_pcg_tables(PcgArgs A, const u
         const long long nf = scan[A.S.c_pref[s + 1]] - b;
         const int cs = chunk_size(nf);
         nch_s[s] = (int)((nf + cs - 1) / cs);
+        csz_s[s] = cs;
         PcgScene& P = A.sc[s];
         P.nf = (int)nf;
         P.csize = cs;
@@ -302,46 +305,55 @@ __global__ void __launch_bounds__(kTableThreads) k_pcg_tables(PcgArgs A, const u
         ordered |= P.ordered;
     }
     const int any_ordered = __syncthreads_or(ordered);
-    const bool may = limit > 0 && !any_ordered && k <= kResMaxScenes;
-    auto cpb_of = [&](int s) { return nch_s[s] > A.res_blocks ? 2 : 1; };  // chunks per block
+    const bool may = A.fast && G > 0 && !any_ordered && k <= kResMaxScenes;
+    auto max_cpb = [&](int s) { return res_max_cpb(A.mode, k, csz_s[s]); };
     auto resident = [&](int s) {
-        return may && nch_s[s] <= limit && res_fits(A.mode, cpb_of(s) * A.sc[s].csize);
+        return may && nch_s[s] <= kResMaxChunks && nch_s[s] <= max_cpb(s) * G;
     };
     if (may) {
         for (int s = threadIdx.x; s < k; s += kTableThreads) {
             int rank = 0;
             for (int t = 0; t < k; ++t) rank += nch_s[t] > nch_s[s] || (nch_s[t] == nch_s[s] && t < s);
             order_s[rank] = s;
+            if (resident(s))
+                for (int q = 0; q < 4; ++q) {
+                    const int c = min(1 << q, max_cpb(s));
+                    atomicAdd(&need_s[res_class(k, csz_s[s])][q], (nch_s[s] + c - 1) / c);
+                }
         }
     }
     __syncthreads();
     if (threadIdx.x != 0) return;
     long long acc = 0;
-    int nstream = 0, partials = 0, groups = 0;
+    int nstream = 0, partials = 0;
     for (int s = 0; s < k; ++s) {
         chp[s] = acc;
         if (resident(s)) continue;
         acc += nch_s[s];
         ++nstream;
-        if (A.res) A.res[s] = make_int4(-1, 0, 0, 0);
+        A.res[s] = make_int4(-1, 0, 0, 0);
     }
     chp[k] = acc;
-    for (int i = 0; may && i < k; ++i) {
-        const int s = order_s[i], nch = nch_s[s], G = A.res_blocks;
-        if (!resident(s)) continue;
-        const int m = (nch + cpb_of(s) - 1) / cpb_of(s);
-        int g = 0;
-        while (g < groups && fill_s[g] + m > G) ++g;
-        if (g == groups) fill_s[groups++] = 0;
-        A.res[s] = make_int4(g * G + fill_s[g], m, nch, partials);
-        A.res_count[32 * s] = 0u;
-        fill_s[g] += m;
-        partials += nch;
+    for (int cls = 0; cls < kResClasses; ++cls) {
+        int groups = 0, q = 0;
+        while (q < 3 && need_s[cls][q] > G) ++q;
+        for (int i = 0; may && i < k; ++i) {
+            const int s = order_s[i], nch = nch_s[s];
+            if (res_class(k, csz_s[s]) != cls || !resident(s)) continue;
+            const int c = min(max(1 << q, (nch + G - 1) / G), max_cpb(s)), m = (nch + c - 1) / c;
+            int g = 0;
+            while (g < groups && fill_s[g] + m > G) ++g;
+            if (g == groups) fill_s[groups++] = 0;
+            A.res[s] = make_int4(g * G + fill_s[g], m, nch, partials);
+            A.res_count[32 * s] = 0u;
+            fill_s[g] += m;
+            partials += nch;
+        }
+        A.ctl->nvirt[cls] = groups * G;
     }
     A.ctl->all_done = 0;
     A.ctl->all_inner_done = 0;
     A.ctl->any_ordered = any_ordered;
-    A.ctl->nvirt = groups * A.res_blocks;
     A.ctl->nstream = nstream;
 }
 
@@ -1351,8 +1363,7 @@ cudaError_t launch_pcg_prepare(const PcgArgs& A, uint32_t* pred, uint32_t* scan,
         k_fl_write<<<grid_for(S.nc), kBlock, 0, st>>>(A, scan);
         count_launch();
     }
-    const int limit = A.fast && A.mode != kRef32 ? res_chunk_limit(A.res_blocks, A.mode) : 0;
-    k_pcg_tables<<<1, kTableThreads, 0, st>>>(A, scan, limit);
+    k_pcg_tables<<<1, kTableThreads, 0, st>>>(A, scan);
     count_launch();
     return cudaGetLastError();
 }
@@ -2272,7 +2283,7 @@ static cudaError_t coop_launch_fast(const PcgArgs& A, int nblocks, cudaStream_t 
     return e;
 }
 
-template <int MODE, int R>
+template <int MODE, int CLASS>
 static cudaError_t coop_launch_res(const PcgArgs& A, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)A.res_blocks);
@@ -2284,8 +2295,18 @@ static cudaError_t coop_launch_res(const PcgArgs& A, cudaStream_t st) {
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, k_pcg_res<MODE, R>, A);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, k_pcg_res<MODE, CLASS>, A);
     count_launch();
+    return e;
+}
+
+template <int MODE>
+static cudaError_t launch_res(const PcgArgs& A, cudaStream_t st) {
+    cudaError_t e = cudaSuccess;
+    if (e == cudaSuccess && (A.classes & 1)) e = coop_launch_res<MODE, 0>(A, st);
+    if (e == cudaSuccess && (A.classes & 2)) e = coop_launch_res<MODE, 1>(A, st);
+    if (e == cudaSuccess && (A.classes & 4)) e = coop_launch_res<MODE, 2>(A, st);
+    if (e == cudaSuccess && (A.classes & 8)) e = coop_launch_res<MODE, 3>(A, st);
     return e;
 }
 
@@ -2296,12 +2317,8 @@ static cudaError_t coop_launch_res(const PcgArgs& A, cudaStream_t st) {
 cudaError_t launch_pcg_solve(const PcgArgs& A, int nblocks, cudaStream_t st) {
     cudaError_t e = cudaSuccess;
     if (A.fast) {
-        const int limit = res_chunk_limit(A.res_blocks, A.mode);
-        if (limit > 0) {
-            e = A.mode == kFp64 ? coop_launch_res<kFp64, 2>(A, st) : coop_launch_res<kMixed, 2>(A, st);
-            if (e == cudaSuccess && !A.all_small)
-                e = A.mode == kFp64 ? coop_launch_res<kFp64, kResRounds>(A, st)
-                                    : coop_launch_res<kMixed, kResRounds>(A, st);
+        if (A.mode != kRef32 && A.res_blocks > 0) {
+            e = A.mode == kFp64 ? launch_res<kFp64>(A, st) : launch_res<kMixed>(A, st);
             if (e != cudaSuccess) return e;
         }
         if (A.mode == kRef32)
@@ -2358,9 +2375,12 @@ int pcg_res_blocks(int device, int mode) {
         return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmem) == cudaSuccess &&
                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, kResThreads, kResSmem) == cudaSuccess && per > 0;
     };
-    const bool ok = mode == kFp64
-                        ? fits((const void*)k_pcg_res<kFp64, 2>) && fits((const void*)k_pcg_res<kFp64, kResRounds>)
-                        : fits((const void*)k_pcg_res<kMixed, 2>) && fits((const void*)k_pcg_res<kMixed, kResRounds>);
+    const void* const f64[] = {(const void*)k_pcg_res<kFp64, 0>, (const void*)k_pcg_res<kFp64, 1>,
+                               (const void*)k_pcg_res<kFp64, 2>, (const void*)k_pcg_res<kFp64, 3>};
+    const void* const f32[] = {(const void*)k_pcg_res<kMixed, 0>, (const void*)k_pcg_res<kMixed, 1>,
+                               (const void*)k_pcg_res<kMixed, 2>, (const void*)k_pcg_res<kMixed, 3>};
+    bool ok = true;
+    for (int c = 0; c < kResClasses; ++c) ok = ok && fits(mode == kFp64 ? f64[c] : f32[c]);
     if (!ok) cudaGetLastError();
     return ok ? sms : 0;  // 0: no scene is resident
 }

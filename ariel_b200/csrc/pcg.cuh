@@ -42,9 +42,8 @@ struct PcgCtl {
     int all_done;
     int all_inner_done;
     int any_ordered;
-    int nvirt;    // block positions of the resident solve (whole groups of gridDim.x)
-    int nstream;  // scenes left to the streaming kernel
-    int pad[3];
+    int nvirt[4];  // block positions of the resident solve's classes (whole groups of gridDim.x)
+    int nstream;   // scenes left to the streaming kernel
 };
 
 struct Barrier {
@@ -79,7 +78,7 @@ struct PcgArgs {
     unsigned* res_count;
     int res_blocks;            // its blocks (one per SM)
     int all_resident;          // every scene fits the resident solve whatever its FLUID count
-    int all_small;             // and has the smallest chunks
+    int classes;               // bit c: some scene may be of class c
     // per-cell operator data (dense over packed cells)
     uint8_t* mask;   // bit d set: neighbour d (-x,+x,-y,+y,-z,+z) is FLUID
     double* diag;    // ADiag (fp32 value for REF32, fp64 otherwise)
@@ -148,13 +147,12 @@ inline long long chunk_bound(long long cells) {
     const long long hi = (cells + kChunkMax - 1) / kChunkMax;
     return std::min(lo, std::max(kChunkTarget, hi));
 }
-// The resident solve: scenes of at most two chunks per block (one block per SM) whose cells fit
-// its shared memory together with slots for neighbours in other blocks, of which bricks of the
+// The resident solve: scenes of one chunk or more per block (one block per SM) whose cells fit its
+// shared memory together with slots for neighbours in other blocks, of which bricks of the
 // FLUID list's order have about 0.6 per cell.
 constexpr int kResMaxChunks = 320;
 constexpr int kResMaxScenes = 128;  // as the streaming fast kernel
 constexpr size_t kResSmem = 225 * 1024;  // all of an SM's but 2 KB for the static part
-inline int res_chunk_limit(int blocks, int mode) { return mode == kRef32 ? 0 : std::min(2 * blocks, kResMaxChunks); }
 // Slots for neighbours in other blocks beside a block's `cells` cells (positions fit 13 bits).
 __host__ __device__ constexpr int res_halo_slots(int mode, int cells) {
     const long long tb = mode == kFp64 ? 8 : 4;
@@ -162,8 +160,25 @@ __host__ __device__ constexpr int res_halo_slots(int mode, int cells) {
     const long long most = 8190 - cells;
     return (int)(left < most ? left : most);
 }
+// Classes of resident scenes, one kernel each, by the rounds of one cell per thread that a chunk
+// takes and the chunks of a half block: a scene alone spreads over as many SMs as it can (one
+// chunk per half); with other scenes small chunks share a block, up to 4,096 cells, so that all
+// scenes iterate side by side (six 32^3-64^3 scenes: one group of blocks instead of four one
+// after another).
+constexpr int kResClasses = 4;
+__host__ __device__ constexpr int res_rounds(int c) { return c == 0 || c == 1 ? 2 : (c == 2 ? 4 : 8); }
+__host__ __device__ constexpr int res_chunks(int c) { return c == 1 ? 4 : (c == 2 ? 2 : 1); }
+__host__ __device__ constexpr int res_class(int scenes, int csize) {
+    return csize <= 512 ? (scenes == 1 ? 0 : 1) : (csize <= 1024 && scenes > 1 ? 2 : 3);
+}
 __host__ __device__ constexpr bool res_fits(int mode, int cells) {
     return 4 * res_halo_slots(mode, cells) >= 3 * cells;
+}
+// Most chunks of `csize` cells that a block takes (0: none fits).
+__host__ __device__ constexpr int res_max_cpb(int mode, int scenes, int csize) {
+    int c = 2 * res_chunks(res_class(scenes, csize));
+    while (c > 0 && !res_fits(mode, c * csize)) c >>= 1;
+    return c;
 }
 constexpr int kBrickMaxCells = 2048;
 constexpr int kBrickMaxExt = 2744;

@@ -31,29 +31,28 @@ __device__ __forceinline__ double4 ldcg4(const double4* p) {
     return make_double4(a.x, a.y, b.x, b.y);
 }
 
-// One block per SM: two halves of kPcgThreads threads, each with a chunk.  Fewer arrivals and
+// One block per SM: two halves of kPcgThreads threads, each with one chunk or more.  Fewer arrivals and
 // pollers make the barrier cheaper than two blocks per SM do (148 against 291 blocks: 2.2 against
 // 2.9 us for an arrival, the wait and the reading of three sums per chunk).
 constexpr int kResThreads = 2 * kPcgThreads;
-constexpr int kResRounds = kChunkMax / kPcgThreads;
 constexpr unsigned kResOut = 0x1fff;  // a neighbour without a slot of u
 static_assert(2 * kChunkMax + 2 * kChunkMax / 2 < (int)kResOut, "positions of u must fit 13 bits");
 
-// One block's part in one scene's solve; R: rounds of one cell per thread (csize <= 256 R).  False
-// when a wait gave up.
-template <int MODE, int R>
+// One block's part in one scene's solve: C chunks per half, Q rounds of one cell per thread in
+// each (csize <= 256 Q).  False when a wait gave up.
+template <int MODE, int Q, int C>
 __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
     using T = typename VT<MODE>::T;
     using T2 = typename V2<T>::type;
     using T4 = typename V4<T>::type;
-    constexpr int kWarps = kPcgThreads / 32;
+    constexpr int R = Q * C, kWarps = kPcgThreads / 32;
     // halo entries of a thread loaded ahead of alpha and beta, in registers
     constexpr int kAhead = R <= 2 ? 2 : (MODE == kFp64 ? 2 : 5);
     const DevState& S = A.S;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int half = tid / kPcgThreads, htid = tid % kPcgThreads, hwid = htid >> 5;
     extern __shared__ __align__(16) unsigned char dyn[];
-    __shared__ double dsum[2][3][kWarps], total[3];
+    __shared__ double dsum[2 * C][3][kWarps], total[3];
     __shared__ int s_nhalo;
     // the scene's solver state, kept by thread 0; the others read alpha, beta and stop
     __shared__ struct {
@@ -66,17 +65,21 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
     const unsigned long long tmo = A.timeout_ns;
     const SceneDev& D = S.scenes[sc];
     const int4 pl = A.res[sc];
-    // this block's first chunk and its chunks (cpb for all blocks but perhaps the last)
-    const int nch = pl.z, cpb = nch > pl.y ? 2 : 1;
-    const int ch0 = (v - pl.x) * cpb, ch = ch0 + half;
-    const bool mine = half < cpb && ch < nch;
+    // this block's first chunk and its chunks (cpb for all blocks but perhaps the last); half h
+    // has the chunks ch0 + h, ch0 + h + 2, ...
+    const int nch = pl.z, cpb = (nch + pl.y - 1) / pl.y;
+    const int ch0 = (v - pl.x) * cpb;
     const int n = D.n;
     const int nf = A.sc[sc].nf, csize = A.sc[sc].csize;
-    // list positions of the block: [t0, t0 + blen); of this half: [base, base + len) from t0
+    // list positions of the block: [t0, t0 + blen)
     const long long t0 = A.fl_pref[sc] + (long long)ch0 * csize;
     const int blen = min(cpb * csize, nf - ch0 * csize);
-    const int base = half * csize;
-    const int len = mine ? min(csize, nf - ch * csize) : 0;
+    // round q of this thread: whether it has a cell, and its position in the block
+    auto cell_of = [&](int q, int& o) -> bool {
+        const int i = htid + (q % Q) * kPcgThreads;
+        o = (half + 2 * (q / Q)) * csize + i;
+        return i < csize && o < blen;
+    };
     // Shared memory: per cell (p, x), the diagonal, pc, u, the cell index and three words of
     // neighbour positions in u (x, y, z pairs of 13 bits; bit 26 of the first: some neighbour
     // lies in another block); u continues with the halo -- the neighbours in other blocks --
@@ -99,27 +102,37 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
     };
     // Publishes the `nsum` sums of this block's chunks and waits for the scene's other blocks
     // (nsum 0: a barrier).  False when the wait gave up.
-    auto arrive_wait = [&](int nsum, double a, double b, double c) -> bool {
+    auto arrive_wait = [&](int nsum, double (&a)[C], double (&b)[C], double (&c)[C]) -> bool {
         ++epoch;
         if (nsum > 0) {
-            a = warp_sum(a);
-            b = warp_sum(b);
-            if (nsum > 2) c = warp_sum(c);
+#pragma unroll
+            for (int j = 0; j < C; ++j) {
+                a[j] = warp_sum(a[j]);
+                b[j] = warp_sum(b[j]);
+                if (nsum > 2) c[j] = warp_sum(c[j]);
+            }
             if (lane == 0) {
-                dsum[half][0][hwid] = a;
-                dsum[half][1][hwid] = b;
-                dsum[half][2][hwid] = c;
+#pragma unroll
+                for (int j = 0; j < C; ++j) {
+                    dsum[half + 2 * j][0][hwid] = a[j];
+                    dsum[half + 2 * j][1][hwid] = b[j];
+                    dsum[half + 2 * j][2][hwid] = c[j];
+                }
             }
         }
         __syncthreads();
         if (hwid < nsum) {
-            // block_sum2's second step: its tree over a warp whose lanes past the eight warp
-            // sums hold zeros
-            double x = lane < kWarps ? dsum[half][hwid][lane] : 0.0;
-            static_assert(kWarps == 8, "three steps sum the warps");
 #pragma unroll
-            for (int o = 4; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-            if (lane == 0 && mine) partial(epoch)[hwid * nch + ch] = x;
+            for (int j = 0; j < C; ++j) {
+                // block_sum2's second step: its tree over a warp whose lanes past the eight warp
+                // sums hold zeros
+                const int i = half + 2 * j;
+                double x = lane < kWarps ? dsum[i][hwid][lane] : 0.0;
+                static_assert(kWarps == 8, "three steps sum the warps");
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+                if (lane == 0 && i < cpb && ch0 + i < nch) partial(epoch)[hwid * nch + ch0 + i] = x;
+            }
         }
         __syncthreads();
         bool ok = true;
@@ -191,7 +204,9 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
         ub[zero] = (T)0;
     }
     __syncthreads();
-    for (int o = base + htid; o < base + len; o += kPcgThreads) {
+    for (int q = 0; q < R; ++q) {
+        int o;
+        if (!cell_of(q, o)) continue;
         const uint4 rc = A.rec[t0 + o];
         const uint32_t c = rc.x, m = rc.y;
         T dg;
@@ -234,22 +249,31 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
     T r[R], w[R], sv[R];
 
     for (int outer = 0;; ++outer) {
-        // ---- residual r = b - A x, |b|^2 ------------------------------------------------
-        double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-        for (int o = base + htid; o < base + len; o += kPcgThreads) {
-            const long long c = cs[o];
-            const double bv = (double)S.D[c];
-            const double xc = __ldcg(S.P64 + c);
-            const double ax = ax_diag<double>(A, D, c, xc, [&](long long q) { return __ldcg(S.P64 + q); });
-            const double rv = bv - ax;
-            if (MODE == kMixed)
-                A.r64[c] = rv;
-            else
-                ((T*)A.r)[c] = (T)rv;
-            a0 += rv * rv;
-            a1 += bv * bv;
-        }
-        if (!arrive_wait(2, a0, a1, 0.0)) return false;
+        // ---- residual r = b - A x, |b|^2 ----------------------------------------------------
+        double a0[C], a1[C], a2[C];
+        auto clear = [&] {
+#pragma unroll
+            for (int j = 0; j < C; ++j) a0[j] = a1[j] = a2[j] = 0.0;
+        };
+        clear();
+#pragma unroll
+        for (int j = 0; j < C; ++j)
+            for (int q = j * Q; q < (j + 1) * Q; ++q) {
+                int o;
+                if (!cell_of(q, o)) break;
+                const long long c = cs[o];
+                const double bv = (double)S.D[c];
+                const double xc = __ldcg(S.P64 + c);
+                const double ax = ax_diag<double>(A, D, c, xc, [&](long long p) { return __ldcg(S.P64 + p); });
+                const double rv = bv - ax;
+                if (MODE == kMixed)
+                    A.r64[c] = rv;
+                else
+                    ((T*)A.r)[c] = (T)rv;
+                a0[j] += rv * rv;
+                a1[j] += bv * bv;
+            }
+        if (!arrive_wait(2, a0, a1, a2)) return false;
         sums(2, [] {}, [&] {
             const double rr = total[0];
             if (outer == 0) st.bb = total[1];
@@ -285,11 +309,11 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
         auto r0 = [&](long long q) -> T {
             return MODE == kMixed ? (T)__ldcg(A.r64 + q) : __ldcg((const T*)A.r + q);
         };
-        a0 = a1 = 0.0;
+        clear();
 #pragma unroll
         for (int q = 0; q < R; ++q) {
-            const int o = base + htid + q * kPcgThreads;
-            if (o < base + len) {
+            int o;
+            if (cell_of(q, o)) {
                 const long long c = cs[o];
                 const uint32_t m = A.mask[c];
                 const T rv = r0(c), pcc = pcs[o];
@@ -309,11 +333,11 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
                 w[q] = wv;
                 sv[q] = (T)0;
                 px[o] = mk2<T>((T)0, xv);
-                a0 += (double)rv * (double)uv;
-                a1 += (double)wv * (double)uv;
+                a0[q / Q] += (double)rv * (double)uv;
+                a1[q / Q] += (double)wv * (double)uv;
             }
         }
-        if (!arrive_wait(2, a0, a1, 0.0)) return false;
+        if (!arrive_wait(2, a0, a1, a2)) return false;
         // ---- iterations: k_pcg_fast's update of (r, w, s, p, x, u), one exchange each ---
         // The halo comes from L2 as its owners' (r, w, s, pc) of the last iteration; the loads
         // are issued as soon as the wait ends, ahead of alpha and beta.
@@ -368,8 +392,8 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
                 ub[cells + h] = u_of(ldcg4(Ac + hcell[h]));
 #pragma unroll
             for (int q = 0; q < R; ++q) {
-                const int o = base + htid + q * kPcgThreads;
-                if (o < base + len) {
+                int o;
+                if (cell_of(q, o)) {
                     const T pc = pcs[o];
                     const T2 b = px[o];
                     const T s1 = w[q] + bt * sv[q];
@@ -384,12 +408,12 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
                 }
             }
             __syncthreads();
-            a0 = a1 = a2 = 0.0;
+            clear();
             auto apply = [&](auto has_out) {
 #pragma unroll
                 for (int q = 0; q < R; ++q) {
-                    const int o = base + htid + q * kPcgThreads;
-                    if (o < base + len) {
+                    int o;
+                    if (cell_of(q, o)) {
                         const uint32_t nb[3] = {nw[o], nw[cells + o], nw[2 * cells + o]};
                         const T un = ub[o];
                         T a = dgs[o] * un;
@@ -408,13 +432,13 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
                             // products of two floats are exact in double, so the fused sums
                             // round as the separate ones
                             const double dr = (double)r[q], du = (double)un;
-                            a0 = __fma_rn(dr, du, a0);
-                            a1 = __fma_rn((double)wn, du, a1);
-                            a2 = __fma_rn(dr, dr, a2);
+                            a0[q / Q] = __fma_rn(dr, du, a0[q / Q]);
+                            a1[q / Q] = __fma_rn((double)wn, du, a1[q / Q]);
+                            a2[q / Q] = __fma_rn(dr, dr, a2[q / Q]);
                         } else {
-                            a0 += (double)r[q] * (double)un;
-                            a1 += (double)wn * (double)un;
-                            a2 += (double)r[q] * (double)r[q];
+                            a0[q / Q] += (double)r[q] * (double)un;
+                            a1[q / Q] += (double)wn * (double)un;
+                            a2[q / Q] += (double)r[q] * (double)r[q];
                         }
                     }
                 }
@@ -428,12 +452,14 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
         __syncthreads();
         if (tid == 0) st.stop = 0;
         // fold the solve's x back: MIXED adds the correction to x64, FP64 stores x64
-        for (int o = base + htid; o < base + len; o += kPcgThreads) {
+        for (int q = 0; q < R; ++q) {
+            int o;
+            if (!cell_of(q, o)) continue;
             const uint32_t c = cs[o];
             S.P64[c] = MODE == kMixed ? S.P64[c] + (double)px[o].y : (double)px[o].y;
         }
         if (MODE != kMixed) break;
-        if (!arrive_wait(0, 0.0, 0.0, 0.0)) return false;
+        if (!arrive_wait(0, a0, a1, a2)) return false;
     }
     if (ch0 == 0 && tid == 0) {
         PcgScene o = load_sc(A.sc + sc);
@@ -459,25 +485,27 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
         Tt.cell_outer += (double)nf * (double)sweeps;
         Tt.not_converged += st.converged ? 0 : 1;
     }
-    for (int o = base + htid; o < base + len; o += kPcgThreads) {
+    for (int q = 0; q < R; ++q) {
+        int o;
+        if (!cell_of(q, o)) continue;
         const uint32_t c = cs[o];
         S.P[c] = (float)S.P64[c];
     }
     return true;
 }
 
-// R = 2 takes the scenes of small chunks, without the code (and its registers) of rounds that none
-// of their threads has; R = kResRounds the others.
-template <int MODE, int R>
+// One kernel per class of scenes (res_class), so that none carries the code and the registers of
+// rounds that its threads do not have.
+template <int MODE, int CLASS>
 __global__ void __launch_bounds__(kResThreads, 1) k_pcg_res(PcgArgs A) {
     if (A.ctl->any_ordered) return;  // the ordered preconditioner runs in k_pcg
     const DevState& S = A.S;
-    const int tid = threadIdx.x, nvirt = A.ctl->nvirt, k = S.k;
+    const int tid = threadIdx.x, nvirt = A.ctl->nvirt[CLASS], k = S.k;
     __shared__ int s_scene;
-    if (R == 2 && blockIdx.x == 0)
+    if (blockIdx.x == 0)
         for (int s = tid; s < k; s += kResThreads) {
             const int4 e = A.res[s];
-            if (e.x < 0 || e.z > 0) continue;
+            if (e.x < 0 || e.z > 0 || res_class(k, A.sc[s].csize) != CLASS) continue;
             // a scene without FLUID cells: solved as it is
             PcgScene o = load_sc(A.sc + s);
             o.outer = MODE == kMixed ? 1 : 0;
@@ -492,11 +520,11 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_res(PcgArgs A) {
         __syncthreads();
         for (int s = tid; s < k; s += kResThreads) {
             const int4 e = A.res[s];
-            if (v >= e.x && v < e.x + e.y && (A.sc[s].csize <= 2 * kPcgThreads) == (R == 2)) s_scene = s;
+            if (v >= e.x && v < e.x + e.y && res_class(k, A.sc[s].csize) == CLASS) s_scene = s;
         }
         __syncthreads();
         const int sc = s_scene;
         if (sc < 0) continue;  // no chunk for this block in this group
-        if (!res_scene<MODE, R>(A, sc, v)) return;
+        if (!res_scene<MODE, res_rounds(CLASS), res_chunks(CLASS)>(A, sc, v)) return;
     }
 }
