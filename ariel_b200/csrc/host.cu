@@ -885,6 +885,7 @@ ariel_status new_sim(const AsimSceneDesc* descs, int k, const AsimParams& prm, c
         for (auto& e : set) cudaEventCreate(&e);
     cudaEventCreate(&s->tb);
     cudaEventCreate(&s->te);
+    host_pool_retain();
     *out = s;
     return ARIEL_OK;
 }
@@ -900,6 +901,7 @@ void delete_sim(ariel_sim* s) {
     cudaEventDestroy(s->te);
     if (s->own_stream) cudaStreamDestroy(s->stream);
     delete s;
+    host_pool_release();
 }
 
 }  // namespace hostimpl
@@ -1311,28 +1313,26 @@ ariel_status ariel_get_particles(ariel_sim* s, int32_t scene, float* pos, float*
     ARIEL_CUDA(cudaStreamSynchronize(s->stream));
     const long long b = s->ppref[scene], n = s->ppref[scene + 1] - b;
     if (n == 0) return ARIEL_OK;
-    std::vector<float4> p4(n), v4(n);
-    ARIEL_CUDA(copy_sync(s->stream, p4.data(), s->S.pos4 + b, n * sizeof(float4), cudaMemcpyDeviceToHost));
-    ARIEL_CUDA(copy_sync(s->stream, v4.data(), s->S.vel4 + b, n * sizeof(float4), cudaMemcpyDeviceToHost));
-    for (long long i = 0; i < n; ++i) {
-        if (pos) {
-            pos[3 * i] = p4[i].x;
-            pos[3 * i + 1] = p4[i].y;
-            pos[3 * i + 2] = p4[i].z;
-        }
-        if (vel) {
-            vel[3 * i] = v4[i].x;
-            vel[3 * i + 1] = v4[i].y;
-            vel[3 * i + 2] = v4[i].z;
-        }
-        if (mass) mass[i] = p4[i].w;
-        if (type) type[i] = type_bits(v4[i]);
+    // two rounds through the I/O staging area: positions and velocities, then mass and type (and
+    // the densities from their own buffer)
+    float* const stage = s->d_stage;
+    if (pos || vel) {
+        ARIEL_CUDA(launch_pack_state(s->S.pos4 + b, s->S.vel4 + b, stage, stage + 3 * n, n, s->stream));
+        std::vector<HostPiece> h;
+        if (pos) h.push_back({pos, stage, 12 * (size_t)n});
+        if (vel) h.push_back({vel, stage + 3 * n, 12 * (size_t)n});
+        ARIEL_CUDA(download(s->stream, h));
     }
-    if (density) {
-        cudaError_t e = launch_scatter_density(s->S, s->d_dens_id, s->stream);
-        if (e != cudaSuccess) return map_cuda_error(e);
-        ARIEL_CUDA(cudaMemcpyAsync(density, s->d_dens_id + b, n * sizeof(float), cudaMemcpyDeviceToHost, s->stream));
-        ARIEL_CUDA(cudaStreamSynchronize(s->stream));
+    if (density || mass || type) {
+        std::vector<HostPiece> h;
+        if (mass || type) ARIEL_CUDA(launch_pack_w(s->S.pos4 + b, s->S.vel4 + b, stage, (int32_t*)(stage + n), n, s->stream));
+        if (mass) h.push_back({mass, stage, 4 * (size_t)n});
+        if (type) h.push_back({type, stage + n, 4 * (size_t)n});
+        if (density) {
+            ARIEL_CUDA(launch_scatter_density(s->S, s->d_dens_id, s->stream));
+            h.push_back({density, s->d_dens_id + b, 4 * (size_t)n});
+        }
+        ARIEL_CUDA(download(s->stream, h));
     }
     return ARIEL_OK;
 }
@@ -1347,7 +1347,7 @@ ariel_status ariel_get_cells(ariel_sim* s, int32_t scene, int32_t* particle_cell
         ARIEL_CUDA(copy_sync(s->stream, key.data(), s->S.key + pb, pn * sizeof(uint32_t), cudaMemcpyDeviceToHost));
         for (long long i = 0; i < pn; ++i) particle_cell[i] = (int32_t)((long long)key[i] - cb);
     }
-    if (cell_count) ARIEL_CUDA(copy_sync(s->stream, cell_count, s->S.count + cb, cn * sizeof(uint32_t), cudaMemcpyDeviceToHost));
+    if (cell_count) ARIEL_CUDA(download(s->stream, {{cell_count, s->S.count + cb, cn * sizeof(uint32_t)}}));
     return ARIEL_OK;
 }
 
@@ -1381,14 +1381,7 @@ ariel_status ariel_get_grid(ariel_sim* s, int32_t scene, int32_t which, void* bu
     ARIEL_TRY(grid_span(s, scene, which, &d, &elems, &esize, &flags));
     if ((size_t)nbytes != elems * esize) return ARIEL_ERR_INVALID_ARG;
     ARIEL_CUDA(cudaStreamSynchronize(s->stream));
-    if (flags) {
-        std::vector<uint8_t> f(elems);
-        ARIEL_CUDA(copy_sync(s->stream, f.data(), d, elems, cudaMemcpyDeviceToHost));
-        int32_t* o = (int32_t*)buf;
-        for (size_t i = 0; i < elems; ++i) o[i] = f[i];
-    } else {
-        ARIEL_CUDA(copy_sync(s->stream, buf, d, elems * esize, cudaMemcpyDeviceToHost));
-    }
+    ARIEL_CUDA(download(s->stream, {{buf, d, flags ? elems : elems * esize, flags}}));
     return ARIEL_OK;
 }
 
@@ -1407,9 +1400,9 @@ ariel_status ariel_set_grid(ariel_sim* s, int32_t scene, int32_t which, const vo
             if (in[i] < 0 || in[i] > 2) return ARIEL_ERR_INVALID_ARG;
             f[i] = (uint8_t)in[i];
         }
-        ARIEL_CUDA(copy_sync(s->stream, d, f.data(), elems, cudaMemcpyHostToDevice));
+        ARIEL_CUDA(upload(s->stream, d, f.data(), elems));
     } else {
-        ARIEL_CUDA(copy_sync(s->stream, d, buf, elems * esize, cudaMemcpyHostToDevice));
+        ARIEL_CUDA(upload(s->stream, d, buf, elems * esize));
     }
     return ARIEL_OK;
 }

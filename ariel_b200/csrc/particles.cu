@@ -971,7 +971,23 @@ __global__ void k_pack_state(const float4* __restrict__ pos4, const float4* __re
     vel[3 * i + 2] = v.z;
 }
 
+__global__ void k_pack_w(const float4* __restrict__ pos4, const float4* __restrict__ vel4, float* mass, int32_t* type,
+                         long long n) {
+    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    mass[i] = pos4[i].w;
+    type[i] = type_of(vel4[i]);
+}
+
 }  // namespace
+
+cudaError_t launch_pack_w(const float4* pos4, const float4* vel4, float* mass, int32_t* type, long long n,
+                          cudaStream_t st) {
+    if (n == 0) return cudaSuccess;
+    k_pack_w<<<grid_for(n), kBlock, 0, st>>>(pos4, vel4, mass, type, n);
+    count_launch();
+    return cudaGetLastError();
+}
 
 cudaError_t launch_unpack_state(float4* pos4, float4* vel4, const float* pos, const float* vel, long long n,
                                 int* err, cudaStream_t st) {

@@ -74,6 +74,9 @@ cudaError_t launch_unpack_state(float4* pos4, float4* vel4, const float* pos, co
                                 int* err, cudaStream_t st);
 cudaError_t launch_pack_state(const float4* pos4, const float4* vel4, float* pos, float* vel, long long n,
                               cudaStream_t st);
+// mass and type of n particles
+cudaError_t launch_pack_w(const float4* pos4, const float4* vel4, float* mass, int32_t* type, long long n,
+                          cudaStream_t st);
 
 // Exclusive scan of n uint32 values into out[0..n] (out[n] = total).  tmp must hold
 // scan_tmp_bytes(n) bytes.

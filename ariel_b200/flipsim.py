@@ -91,11 +91,11 @@ class Batch:
 
     def get_particles(self, scene=0):
         n = self.count(scene)
-        pos = np.zeros((n, 3), np.float32)
-        vel = np.zeros((n, 3), np.float32)
-        den = np.zeros(n, np.float32)
-        mass = np.zeros(n, np.float32)
-        typ = np.zeros(n, np.int32)
+        pos = np.empty((n, 3), np.float32)
+        vel = np.empty((n, 3), np.float32)
+        den = np.empty(n, np.float32)
+        mass = np.empty(n, np.float32)
+        typ = np.empty(n, np.int32)
         check(self.L.ariel_get_particles(self.h, scene, _p(pos), _p(vel), _p(den), _p(mass), _p(typ)),
               "ariel_get_particles")
         return dict(pos=pos, vel=vel, density=den, mass=mass, type=typ)
@@ -114,14 +114,14 @@ class Batch:
     def get_cells(self, scene=0):
         n = self.count(scene)
         d = self.dim(scene)
-        pc = np.zeros(n, np.int32)
-        cc = np.zeros(d ** 3, np.int32)
+        pc = np.empty(n, np.int32)
+        cc = np.empty(d ** 3, np.int32)
         check(self.L.ariel_get_cells(self.h, scene, _p(pc), _p(cc)), "ariel_get_cells")
         return pc, cc
 
     def get_grid(self, which, scene=0):
         shape, dt = grid_shape(self.dim(scene), which)
-        a = np.zeros(shape, dt)
+        a = np.empty(shape, dt)
         check(self.L.ariel_get_grid(self.h, scene, which, _p(a), a.nbytes), "ariel_get_grid")
         return a
 
@@ -165,7 +165,7 @@ class Batch:
         """The liquid surface's level set ((n+5)^3 samples, sample (i,j,k) at grid point
         (i-2, j-2, k-2))."""
         N = self.dim(scene) + 5
-        phi = np.zeros((N, N, N), np.float32)
+        phi = np.empty((N, N, N), np.float32)
         check(self.L.ariel_get_level_set(self.h, scene, _p(phi), phi.nbytes), "ariel_get_level_set")
         return phi
 
