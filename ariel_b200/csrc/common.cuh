@@ -22,6 +22,11 @@ namespace ariel {
 constexpr int kMaxScenes = 1024;
 constexpr int kBlock = 256;
 
+// Division of a squared distance by a kernel radius squared hh: exactly by its reciprocal where hh
+// is a power of two; by its rounded reciprocal with one correction; as written (hh so large or
+// small that the correction could over- or underflow).
+enum { kDivPow2 = 0, kDivFixed = 1, kDivPlain = 2 };
+
 struct SceneDev {
     int n;             // cells per axis
     int n_forces;
@@ -50,7 +55,7 @@ struct SceneDev {
     int reseed_min, reseed_max;  // particle-count bounds of the reseeding pass
     // When a kernel radius squared (in float) is a power of two, r2 / (h*h) equals
     // r2 * (1 / (h*h)) exactly, so the division can be replaced by a multiplication.
-    int dens_pow2;       // dens_h * dens_h is a power of two
+    int dens_div;        // how r2 / (dens_h * dens_h) is evaluated (kDiv*)
     float dens_inv_hh;
     int re_pow2;         // resample_re^2 is a power of two
     float re_inv_hh;

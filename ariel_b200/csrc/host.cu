@@ -216,6 +216,8 @@ long long layout_bytes(const Layout& L) {
     add(np, 16);  // spos4
     add(np, 16);  // svel4
     add(np, 16);  // gpos4
+    add(nc + 1, 4);  // pstart
+    add(pair_bound(np, nc), 32);  // spair
     add(np, 4);   // dens
     add(np, 4);   // dens by id
     add(6 * np, 4);  // host I/O staging
@@ -457,7 +459,9 @@ SceneDev make_scene(const AsimSceneDesc& d, const AsimParams& p) {
     D.inv_n1 = 1.0 / (dn + 1.0);
     D.inv_nn = 1.0 / (dn * dn);
     D.inv_nn1 = 1.0 / (dn * (dn + 1.0));
-    D.dens_pow2 = pow2(D.dens_h * D.dens_h, &D.dens_inv_hh);
+    const float dens_hh = D.dens_h * D.dens_h;
+    D.dens_div = pow2(dens_hh, &D.dens_inv_hh) ? kDivPow2
+                 : (dens_hh > 0x1p-60f && dens_hh < 0x1p60f) ? kDivFixed : kDivPlain;
     D.re_pow2 = pow2(D.resample_re * D.resample_re, &D.re_inv_hh);
     return D;
 }
@@ -574,6 +578,8 @@ ariel_status build_state(ariel_sim* s, std::vector<HostParticles>& hp, const ari
     ARIEL_TRY(dalloc(s, &S.spos4, np));
     ARIEL_TRY(dalloc(s, &S.svel4, np));
     ARIEL_TRY(dalloc(s, &S.gpos4, np));
+    ARIEL_TRY(dalloc(s, &S.pstart, nc + 1));
+    ARIEL_TRY(dalloc(s, &S.spair, 2 * (size_t)pair_bound(np, nc)));
     ARIEL_TRY(dalloc(s, &S.dens, np));
     ARIEL_TRY(dalloc(s, &s->d_dens_id, np));
     ARIEL_TRY(dalloc(s, &s->d_stage, 6 * (size_t)np));
@@ -845,6 +851,7 @@ ariel_status refresh_scene_table(ariel_sim* s) {
 
 ariel_status sort_and_classify_init(ariel_sim* s) {
     cudaError_t e = launch_sort(s->S, s->scan_tmp, s->stream);
+    s->pairs_stale = false;
     if (e == cudaSuccess) e = launch_fill_dens(s->S, 10.0f, s->stream);  // AddLiquidParticle: m_density = 10
     if (e == cudaSuccess) e = launch_classify(s->S, 1, s->stream);
     if (e != cudaSuccess) return map_cuda_error(e);
@@ -922,8 +929,15 @@ ariel_status enqueue_stage(ariel_sim* s, int g, cudaEvent_t* evs = nullptr) {
     cudaError_t e = cudaSuccess;
     switch (g) {
         case ARIEL_STAGE_BEGIN: e = launch_begin(S, st); break;
-        case ARIEL_STAGE_SORT: e = launch_sort(S, s->scan_tmp, st); break;
-        case ARIEL_STAGE_DENSITY: e = launch_density(S, st); break;
+        case ARIEL_STAGE_SORT:
+            e = launch_sort(S, s->scan_tmp, st);
+            s->pairs_stale = false;
+            break;
+        case ARIEL_STAGE_DENSITY:
+            if (s->pairs_stale) e = launch_make_pairs(S, s->scan_tmp, st);
+            s->pairs_stale = false;
+            if (e == cudaSuccess) e = launch_density(S, st);
+            break;
         case ARIEL_STAGE_FORCES: e = launch_forces(S, st); break;
         case ARIEL_STAGE_P2G: e = launch_p2g(S, s->prm.p2g_faces, st); break;
         case ARIEL_STAGE_CLASSIFY: e = launch_classify(S, 0, st); break;
@@ -936,7 +950,10 @@ ariel_status enqueue_stage(ariel_sim* s, int g, cudaEvent_t* evs = nullptr) {
         case ARIEL_STAGE_GRADIENT: e = launch_gradient(S, st); break;
         case ARIEL_STAGE_EXTRAPOLATE: e = launch_extrapolate(S, st); break;
         case ARIEL_STAGE_G2P_ADVECT: e = launch_g2p_advect(S, st); break;
-        case ARIEL_STAGE_RESAMPLE: e = launch_resample(S, s->scan_tmp, st); break;
+        case ARIEL_STAGE_RESAMPLE:
+            e = launch_resample(S, s->scan_tmp, st);
+            s->pairs_stale = true;
+            break;
         default: return ARIEL_ERR_INVALID_ARG;
     }
     if (e != cudaSuccess) return map_cuda_error(e, "stage launch");
@@ -1102,6 +1119,7 @@ ariel_status step_async(ariel_sim* s) {
         }
     }
     for (auto& f : s->frames) f++;
+    s->pairs_stale = true;  // a replayed step's last sort, too
     return ARIEL_OK;
 }
 

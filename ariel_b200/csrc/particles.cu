@@ -14,6 +14,8 @@ namespace ariel {
 
 namespace {
 
+constexpr float kFar = 1.0e30f;  // out of every kernel's reach
+
 #define SCENE_PREFIX(pref_src)                       \
     __shared__ long long pref_s[kMaxScenes + 1];     \
     load_prefix<kMaxScenes>(pref_s, (pref_src), S.k)
@@ -264,18 +266,49 @@ __global__ void __launch_bounds__(32 * kBigWarps) k_sort_big(DevState S, const u
     }
 }
 
+// The density's pair records: every second slot of a cell writes the pair that starts with it.  `p`
+// is the slot's position; the next one's comes from the next lane (all lanes of the warp call
+// this) or, for the last lane, from next_pos(slot).
+template <class F>
+__device__ __forceinline__ void write_pairs(const DevState& S, const SceneDev& D, bool in, long long s, float4 p,
+                                            F&& next_pos) {
+    float4 q;
+    q.x = __shfl_down_sync(0xffffffffu, p.x, 1);
+    q.y = __shfl_down_sync(0xffffffffu, p.y, 1);
+    q.z = __shfl_down_sync(0xffffffffu, p.z, 1);
+    q.w = __shfl_down_sync(0xffffffffu, p.w, 1);
+    if (!in) return;
+    const int n = D.n;
+    const long long c = D.c_begin + ((long long)cell_coord(D.maxd, p.x) * n + cell_coord(D.maxd, p.y)) * n +
+                        cell_coord(D.maxd, p.z);
+    const uint32_t a = S.start[c], r = (uint32_t)s - a;
+    if (r & 1u) return;
+    if (s + 1 >= S.start[c + 1])
+        q = make_float4(kFar, kFar, kFar, 0.0f);
+    else if ((threadIdx.x & 31) == 31)
+        q = next_pos(s + 1);
+    float4* const rec = S.spair + 2 * (size_t)(S.pstart[c] + r / 2);
+    rec[0] = make_float4(p.x, q.x, p.y, q.y);
+    rec[1] = make_float4(p.z, q.z, p.w, q.w);
+}
+
+template <bool PAIRS>
 __global__ void k_sort_permute(DevState S) {
     SCENE_PREFIX(S.p_pref);
     long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S.np) return;
-    uint32_t g = S.sid[s];
-    float4 p = S.pos4[g];
+    const bool in = s < S.np;
+    if (!PAIRS && !in) return;
+    const SceneDev& D = S.scenes[find_scene(pref_s, S.k, in ? s : 0)];
+    const uint32_t g = in ? S.sid[s] : 0u;
+    const float4 p = in ? S.pos4[g] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (PAIRS) write_pairs(S, D, in, s, p, [&](long long t) { return S.pos4[S.sid[t]]; });
+    if (!in) return;
     float4 v = S.vel4[g];
     S.spos4[s] = p;
     S.svel4[s] = v;
     // SplatParticlesToMACGrid's clamped grid position (particlegridoperations.inl:172-174);
     // non-FLUID particles are placed out of every face's reach (they are skipped, :170)
-    const float maxd = S.scenes[find_scene(pref_s, S.k, s)].maxd;
+    const float maxd = D.maxd;
     float4 gp;
     if (type_of(v) == ARIEL_FLUID) {
         gp.x = gmax(0.0f, gmin(maxd, maxd * p.x));
@@ -283,58 +316,135 @@ __global__ void k_sort_permute(DevState S) {
         gp.z = gmax(0.0f, gmin(maxd, maxd * p.z));
         gp.w = p.w;
     } else {
-        gp = make_float4(1.0e30f, 1.0e30f, 1.0e30f, 0.0f);
+        gp = make_float4(kFar, kFar, kFar, 0.0f);
     }
     S.gpos4[s] = gp;
 }
 
-// ------------------------------------------------------------------------------------------
-// FlipSim::ComputeDensity (flip.cpp:697-733): one thread per slot, 27-cell gather.
-// ------------------------------------------------------------------------------------------
-// weightsum over slots [a, b) in slot order, with the Smooth kernel's division either exact
-// (POW2: h^2 a power of two, so r2 / h^2 == r2 * inv_hh) or as written.
-template <bool POW2>
-__device__ __forceinline__ float density_run(const float4* __restrict__ sp, uint32_t a, uint32_t b, float px,
-                                             float py, float pz, float hk, float inv_hh, float weightsum) {
-    const float2 nxy = make_float2(-px, -py);
-#pragma unroll 4
-    for (uint32_t t = a; t < b; ++t) {
-        const float4 q = sp[t];
-        const float sqd = sqrlength_xy2(q, nxy, pz);
-        const float weight = q.w * (POW2 ? gmax(1.0f - sqd * inv_hh, 0.0f) : smooth_k(sqd, hk));
-        weightsum = weightsum + weight;
-    }
-    return weightsum;
+// The pair records of slots sorted without them (the resampler's Sort).
+__global__ void k_make_pairs(DevState S) {
+    SCENE_PREFIX(S.p_pref);
+    const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool in = s < S.np;
+    const SceneDev& D = S.scenes[find_scene(pref_s, S.k, in ? s : 0)];
+    write_pairs(S, D, in, s, in ? S.spos4[s] : make_float4(0.0f, 0.0f, 0.0f, 0.0f),
+                [&](long long t) { return S.spos4[t]; });
 }
 
-// At most 40 registers (three 512-thread blocks per SM): the issue-bound gather gains from the
-// extra resident warps more than it loses to an 8-byte spill (5-6% faster measured).
-__global__ void __launch_bounds__(512, 3) k_density(DevState S) {
-    SCENE_PREFIX(S.p_pref);
-    long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S.np) return;
-    const SceneDev& D = S.scenes[find_scene(pref_s, S.k, s)];
-    float4 p = S.spos4[s];
-    if (type_of(S.svel4[s]) == ARIEL_SOLID) {
-        S.dens[s] = 1.0f;
-        return;
+// ------------------------------------------------------------------------------------------
+// FlipSim::ComputeDensity (flip.cpp:697-733): a 27-cell gather, one thread per pair of a cell's
+// particles.
+//
+// The kernel radius is 2 cells, so nearly all of the 27 cells' 216 particles count.  One particle
+// per thread reading one 16-byte record per candidate was bound by what L1 returns to the
+// registers (86% of its wavefronts; a warp's 16-byte loads take four however many lanes share
+// an address).  Here a thread takes the two particles of a pair -- the same cell, so the same
+// candidates -- and reads the candidates two at a time as the records k_sort_permute pairs up:
+// a quarter of the records per pair of particles, and their terms as packed fp32x2 operations,
+// one candidate per lane of the pair.  Each particle's sum still adds its candidates one by one in
+// slot order, with the bits of the scalar expressions; the far second particle of an odd pair
+// adds +0.  128^3 dam break 0.645 -> 0.53 ms, 64^3 0.100 -> 0.082, 77^3 (no power of two) 0.248 ->
+// 0.168, with 0.03 ms (128^3) more in the sort; now bound by the fp32 pipe, 12 operations a
+// candidate.  Four or three blocks per SM measure the same, five 2-10% slower; unrolled by 4 2%
+// slower, not at all 4%.
+// ------------------------------------------------------------------------------------------
+__device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
+// glm::max(x, 0.0f) for x = 1 - q (never -0), NaN kept as the ternary keeps it
+__device__ __forceinline__ float max0_nan(float x) {
+    float r;
+    asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float min_nan(float x, float y) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(y));
+    return r;
+}
+
+// One target against a pair of candidates (x, y, z, masses m): their Smooth weights.
+// kDivPow2: the radius squared hh is a power of two, so r2 / hh == r2 * inv exactly.  kDivFixed: the
+// quotient estimate r2 * inv, inv the rounded 1 / hh, is corrected by its exact remainder, which
+// gives the correctly rounded quotient (Markstein, IBM J. Res. Dev. 34, 1990) -- checked against
+// the division for every r2 up to 8 hh at 40 grid sizes.  r2 is held to 8 hh (weight 0, as beyond
+// it) so that the remainder of an infinite one is no NaN; a remainder that underflows changes
+// quotients below 2^-70, which 1 - q does not see.
+// kDivPlain (radii out of any scene's range): the division.
+// The assembler contracts a packed multiply that feeds a packed add into one rounding, whatever
+// --fmad says, so such products are fused adds of `nzero`, a -0 that it cannot see through.
+template <int DIV>
+__device__ __forceinline__ float2 smooth_pair(float2 x, float2 y, float2 z, float2 m, float2 nx, float2 ny, float2 nz,
+                                              float hh, float ninv, float2 nzero) {
+    const float2 dx = __fadd2_rn(x, nx), dy = __fadd2_rn(y, ny), dz = __fadd2_rn(z, nz);
+    float2 r2 = __fadd2_rn(__fadd2_rn(__ffma2_rn(dx, dx, nzero), __ffma2_rn(dy, dy, nzero)),
+                           __ffma2_rn(dz, dz, nzero));
+    float2 nq;  // -(r2 / hh)
+    if (DIV == kDivPow2) {
+        nq = __ffma2_rn(r2, dup2(ninv), nzero);
+    } else if (DIV == kDivPlain) {
+        nq = make_float2(-(r2.x / hh), -(r2.y / hh));
+    } else {
+        r2.x = min_nan(r2.x, 8.0f * hh);
+        r2.y = min_nan(r2.y, 8.0f * hh);
+        nq = __fmul2_rn(r2, dup2(ninv));
+        nq = __ffma2_rn(__ffma2_rn(dup2(hh), nq, r2), dup2(ninv), nq);
     }
+    float2 w = __fadd2_rn(dup2(1.0f), nq);
+    w.x = max0_nan(w.x);
+    w.y = max0_nan(w.y);
+    return __fmul2_rn(m, w);
+}
+
+template <int DIV>
+__device__ __forceinline__ void density_run(const float4* __restrict__ sp, uint32_t a, uint32_t b, const float2 (&n0)[3],
+                                            const float2 (&n1)[3], float hh, float ninv, float2 nzero, float& sum0,
+                                            float& sum1) {
+#pragma unroll 2
+    for (uint32_t t = a; t < b; ++t) {
+        const float4 u = sp[2 * (size_t)t], v = sp[2 * (size_t)t + 1];
+        const float2 x = make_float2(u.x, u.y), y = make_float2(u.z, u.w), z = make_float2(v.x, v.y),
+                     m = make_float2(v.z, v.w);
+        const float2 w0 = smooth_pair<DIV>(x, y, z, m, n0[0], n0[1], n0[2], hh, ninv, nzero);
+        const float2 w1 = smooth_pair<DIV>(x, y, z, m, n1[0], n1[1], n1[2], hh, ninv, nzero);
+        sum0 = sum0 + w0.x;
+        sum0 = sum0 + w0.y;
+        sum1 = sum1 + w1.x;
+        sum1 = sum1 + w1.y;
+    }
+}
+
+constexpr int kDensityBlock = 256;
+__global__ void __launch_bounds__(kDensityBlock, 4) k_density(DevState S, float neg_zero) {
+    __shared__ long long pref_s[kMaxScenes + 1];  // pair begins of the scenes
+    for (int i = threadIdx.x; i <= S.k; i += blockDim.x) pref_s[i] = S.pstart[S.c_pref[i]];
+    __syncthreads();
+    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= pref_s[S.k]) return;
+    const SceneDev& D = S.scenes[find_scene(pref_s, S.k, p)];
+    const float4 u = S.spair[2 * p], v = S.spair[2 * p + 1];
     const int n = D.n;
-    const float hk = D.dens_h;
-    int ci = cell_coord(D.maxd, p.x), cj = cell_coord(D.maxd, p.y), ck = cell_coord(D.maxd, p.z);
-    int z0 = max(ck - 1, 0), z1 = min(ck + 1, n - 1);
-    float weightsum = 0.0f;
-    for (int sx = ci - 1; sx <= ci + 1; ++sx) {
-        if (sx < 0 || sx > n - 1) continue;
-        for (int sy = cj - 1; sy <= cj + 1; ++sy) {
-            if (sy < 0 || sy > n - 1) continue;
-            long long cb = D.c_begin + ((long long)sx * n + sy) * n;
-            uint32_t a = S.start[cb + z0], b = S.start[cb + z1 + 1];
-            weightsum = D.dens_pow2 ? density_run<true>(S.spos4, a, b, p.x, p.y, p.z, hk, D.dens_inv_hh, weightsum)
-                                    : density_run<false>(S.spos4, a, b, p.x, p.y, p.z, hk, D.dens_inv_hh, weightsum);
+    const int ci = cell_coord(D.maxd, u.x), cj = cell_coord(D.maxd, u.z), ck = cell_coord(D.maxd, v.x);
+    const long long c = D.c_begin + ((long long)ci * n + cj) * n + ck;
+    const uint32_t s0 = S.start[c] + 2u * ((uint32_t)p - S.pstart[c]);
+    const bool two = s0 + 1 < S.start[c + 1];
+    const float2 n0[3] = {dup2(-u.x), dup2(-u.z), dup2(-v.x)}, n1[3] = {dup2(-u.y), dup2(-u.w), dup2(-v.y)};
+    const float hh = D.dens_h * D.dens_h, ninv = -D.dens_inv_hh;
+    const float2 nzero = dup2(neg_zero);
+    const int z0 = max(ck - 1, 0), z1 = min(ck + 1, n - 1);
+    float sum0 = 0.0f, sum1 = 0.0f;
+    for (int sx = max(ci - 1, 0); sx <= min(ci + 1, n - 1); ++sx)
+        for (int sy = max(cj - 1, 0); sy <= min(cj + 1, n - 1); ++sy) {
+            const long long cb = D.c_begin + ((long long)sx * n + sy) * n;
+            const uint32_t a = S.pstart[cb + z0], b = S.pstart[cb + z1 + 1];
+            if (D.dens_div == kDivPow2)
+                density_run<kDivPow2>(S.spair, a, b, n0, n1, hh, ninv, nzero, sum0, sum1);
+            else if (D.dens_div == kDivFixed)
+                density_run<kDivFixed>(S.spair, a, b, n0, n1, hh, ninv, nzero, sum0, sum1);
+            else
+                density_run<kDivPlain>(S.spair, a, b, n0, n1, hh, ninv, nzero, sum0, sum1);
         }
-    }
-    S.dens[s] = weightsum / D.max_density;
+    const float md = D.max_density;
+    S.dens[s0] = type_of(S.svel4[s0]) == ARIEL_SOLID ? 1.0f : sum0 / md;
+    if (two) S.dens[s0 + 1] = type_of(S.svel4[s0 + 1]) == ARIEL_SOLID ? 1.0f : sum1 / md;
 }
 
 __global__ void k_fill_dens(DevState S, float v) {
@@ -1018,13 +1128,14 @@ cudaError_t launch_begin(const DevState& S, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-static cudaError_t sort_core(const DevState& S, void* scan_tmp, cudaStream_t st) {
+static cudaError_t sort_core(const DevState& S, void* scan_tmp, bool pairs, cudaStream_t st) {
     cudaMemsetAsync(S.count, 0, sizeof(uint32_t) * (size_t)S.nc, st);
     if (S.np > 0) {
         k_sort_key<<<grid_for(S.np), kBlock, 0, st>>>(S);
         count_launch();
     }
-    cudaError_t e = launch_scan_u32(S.count, S.start, S.nc, scan_tmp, st);
+    cudaError_t e = pairs ? launch_scan_pairs(S.count, S.start, S.pstart, S.nc, scan_tmp, st)
+                          : launch_scan_u32(S.count, S.start, S.nc, scan_tmp, st);
     if (e != cudaSuccess) return e;
     if (S.np > 0) {
         // the scan's scratch is free again: its first word counts the cells for k_sort_big
@@ -1033,20 +1144,29 @@ static cudaError_t sort_core(const DevState& S, void* scan_tmp, cudaStream_t st)
         cudaMemsetAsync(nbig, 0, sizeof(uint32_t), st);
         k_sort_cells<<<grid_for(S.nc), kBlock, 0, st>>>(S, nbig);
         k_sort_big<<<kSortBigBlocks, 32 * kBigWarps, 0, st>>>(S, nbig);
-        k_sort_permute<<<grid_for(S.np), kBlock, 0, st>>>(S);
+        if (pairs)
+            k_sort_permute<true><<<grid_for(S.np), kBlock, 0, st>>>(S);
+        else
+            k_sort_permute<false><<<grid_for(S.np), kBlock, 0, st>>>(S);
         count_launch(4);
     }
     return cudaGetLastError();
 }
 
-cudaError_t launch_sort(const DevState& S, void* scan_tmp, cudaStream_t st) { return sort_core(S, scan_tmp, st); }
+cudaError_t launch_sort(const DevState& S, void* scan_tmp, cudaStream_t st) { return sort_core(S, scan_tmp, true, st); }
+
+cudaError_t launch_make_pairs(const DevState& S, void* scan_tmp, cudaStream_t st) {
+    if (S.np == 0) return cudaSuccess;
+    cudaError_t e = launch_scan_pairs(S.count, S.start, S.pstart, S.nc, scan_tmp, st);
+    if (e != cudaSuccess) return e;
+    k_make_pairs<<<grid_for(S.np), kBlock, 0, st>>>(S);
+    count_launch();
+    return cudaGetLastError();
+}
 
 cudaError_t launch_density(const DevState& S, cudaStream_t st) {
     if (S.np == 0) return cudaSuccess;
-    // 512 threads: measured faster than 256 for this kernel alone (0.79 vs 0.90 ms at 128^3);
-    // the kernel's launch bounds assume this block size
-    constexpr int kDensityBlock = 512;
-    k_density<<<grid_for(S.np, kDensityBlock), kDensityBlock, 0, st>>>(S);
+    k_density<<<grid_for(pair_bound(S.np, S.nc), kDensityBlock), kDensityBlock, 0, st>>>(S, -0.0f);
     count_launch();
     return cudaGetLastError();
 }
@@ -1101,7 +1221,8 @@ cudaError_t launch_g2p_advect(const DevState& S, cudaStream_t st) {
 cudaError_t launch_resample(const DevState& S, void* scan_tmp, cudaStream_t st) {
     // StoreTempParticleVelocities before the resampler (flip.cpp:119) needs no copy: the
     // resampler's constraint check reads pt/ut from the slot copies of its own Sort.
-    cudaError_t e = sort_core(S, scan_tmp, st);
+    // (without the density's pair records, which nothing after it reads)
+    cudaError_t e = sort_core(S, scan_tmp, false, st);
     if (e != cudaSuccess) return e;
     if (S.np == 0) return cudaSuccess;
     k_resample_spring<<<grid_for(S.np), kBlock, 0, st>>>(S);

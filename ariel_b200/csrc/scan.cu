@@ -14,11 +14,12 @@ constexpr int kScanThreads = 256;
 constexpr int kScanItems = 16;
 constexpr int kTile = kScanThreads * kScanItems;
 
-__device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
+template <class T>
+__device__ __forceinline__ T warp_incl_scan(T v) {
     const unsigned lane = threadIdx.x & 31;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        uint32_t t = __shfl_up_sync(0xffffffffu, v, o);
+        T t = __shfl_up_sync(0xffffffffu, v, o);
         if (lane >= (unsigned)o) v += t;
     }
     return v;
@@ -26,49 +27,66 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
 
 // Block-wide exclusive scan of one value per thread; returns the exclusive prefix and the
 // block total through *total.
-__device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* total) {
-    __shared__ uint32_t warp_sums[kScanThreads / 32];
+template <class T>
+__device__ __forceinline__ T block_excl_scan(T v, T* total) {
+    __shared__ T warp_sums[kScanThreads / 32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    uint32_t inc = warp_incl_scan(v);
+    T inc = warp_incl_scan(v);
     if (lane == 31) warp_sums[wid] = inc;
     __syncthreads();
     if (wid == 0) {
         constexpr int kWarps = kScanThreads / 32;
-        uint32_t w = lane < kWarps ? warp_sums[lane] : 0;
+        T w = lane < kWarps ? warp_sums[lane] : 0;
         __syncwarp();
-        uint32_t wi = warp_incl_scan(w);
+        T wi = warp_incl_scan(w);
         if (lane < kWarps) warp_sums[lane] = wi - w;
         if (lane == kWarps - 1) *total = wi;
     }
     __syncthreads();
-    uint32_t r = warp_sums[wid] + inc - v;
+    T r = warp_sums[wid] + inc - v;
     __syncthreads();
     return r;
 }
 
-__global__ void k_tile_sums(const uint32_t* __restrict__ in, long long n, uint32_t* __restrict__ sums) {
+// What is summed for one count: the count itself, or with it, in the upper half of 64 bits, the
+// pairs that hold it (the sort's scan: both prefixes in one pass over the counts).
+__device__ __forceinline__ void widen(uint32_t v, uint32_t& t) { t = v; }
+__device__ __forceinline__ void widen(uint32_t v, unsigned long long& t) {
+    t = (unsigned long long)((v + 1u) >> 1) << 32 | v;
+}
+__device__ __forceinline__ void put(uint32_t* out, uint32_t*, long long i, uint32_t t) { out[i] = t; }
+__device__ __forceinline__ void put(uint32_t* out, uint32_t* pairs, long long i, unsigned long long t) {
+    out[i] = (uint32_t)t;
+    pairs[i] = (uint32_t)(t >> 32);
+}
+
+template <class T>
+__global__ void k_tile_sums(const uint32_t* __restrict__ in, long long n, T* __restrict__ sums) {
     long long base = (long long)blockIdx.x * kTile;
-    uint32_t acc = 0;
+    T acc = 0;
 #pragma unroll
     for (int it = 0; it < kScanItems; ++it) {
         long long i = base + (long long)it * kScanThreads + threadIdx.x;
-        if (i < n) acc += in[i];
+        T t = 0;
+        if (i < n) widen(in[i], t);
+        acc += t;
     }
-    __shared__ uint32_t tot;
+    __shared__ T tot;
     block_excl_scan(acc, &tot);
     if (threadIdx.x == 0) sums[blockIdx.x] = tot;
 }
 
-__global__ void k_scan_sums(uint32_t* sums, long long nt) {
-    __shared__ uint32_t carry_s;
+template <class T>
+__global__ void k_scan_sums(T* sums, long long nt) {
+    __shared__ T carry_s;
     if (threadIdx.x == 0) carry_s = 0;
     __syncthreads();
     for (long long b = 0; b < nt; b += kScanThreads) {
         long long i = b + threadIdx.x;
-        uint32_t v = i < nt ? sums[i] : 0;
-        __shared__ uint32_t tot;
-        uint32_t ex = block_excl_scan(v, &tot);
-        uint32_t carry = carry_s;
+        T v = i < nt ? sums[i] : 0;
+        __shared__ T tot;
+        T ex = block_excl_scan(v, &tot);
+        T carry = carry_s;
         if (i < nt) sums[i] = carry + ex;
         __syncthreads();
         if (threadIdx.x == 0) carry_s = carry + tot;
@@ -77,26 +95,44 @@ __global__ void k_scan_sums(uint32_t* sums, long long nt) {
     if (threadIdx.x == 0) sums[nt] = carry_s;
 }
 
-__global__ void k_tile_scan(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, long long n,
-                            const uint32_t* __restrict__ sums, long long nt) {
+template <class T>
+__global__ void k_tile_scan(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, uint32_t* __restrict__ pairs,
+                            long long n, const T* __restrict__ sums, long long nt) {
     long long base = (long long)blockIdx.x * kTile + (long long)threadIdx.x * kScanItems;
-    uint32_t vals[kScanItems];
-    uint32_t acc = 0;
+    T vals[kScanItems];
+    T acc = 0;
 #pragma unroll
     for (int it = 0; it < kScanItems; ++it) {
         long long i = base + it;
-        vals[it] = i < n ? in[i] : 0;
+        vals[it] = 0;
+        if (i < n) widen(in[i], vals[it]);
         acc += vals[it];
     }
-    __shared__ uint32_t tot;
-    uint32_t ex = block_excl_scan(acc, &tot) + sums[blockIdx.x];
+    __shared__ T tot;
+    T ex = block_excl_scan(acc, &tot) + sums[blockIdx.x];
 #pragma unroll
     for (int it = 0; it < kScanItems; ++it) {
         long long i = base + it;
-        if (i < n) out[i] = ex;
+        if (i < n) put(out, pairs, i, ex);
         ex += vals[it];
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = sums[nt];
+    if (blockIdx.x == 0 && threadIdx.x == 0) put(out, pairs, n, sums[nt]);
+}
+
+template <class T>
+cudaError_t scan(const uint32_t* in, uint32_t* out, uint32_t* pairs, long long n, void* tmp, cudaStream_t st) {
+    long long nt = (n + kTile - 1) / kTile;
+    T* sums = (T*)tmp;
+    if (nt == 0) {
+        cudaMemsetAsync(out, 0, sizeof(uint32_t), st);
+        if (pairs) cudaMemsetAsync(pairs, 0, sizeof(uint32_t), st);
+        return cudaGetLastError();
+    }
+    k_tile_sums<T><<<(unsigned)nt, kScanThreads, 0, st>>>(in, n, sums);
+    k_scan_sums<T><<<1, kScanThreads, 0, st>>>(sums, nt);
+    k_tile_scan<T><<<(unsigned)nt, kScanThreads, 0, st>>>(in, out, pairs, n, sums, nt);
+    count_launch(3);
+    return cudaGetLastError();
 }
 
 std::atomic<long long> g_launches{0};
@@ -105,20 +141,15 @@ std::atomic<long long> g_launches{0};
 void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 long long launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
-size_t scan_tmp_bytes(long long n) { return sizeof(uint32_t) * (size_t)((n + kTile - 1) / kTile + 2); }
+size_t scan_tmp_bytes(long long n) { return sizeof(uint64_t) * (size_t)((n + kTile - 1) / kTile + 2); }
 
 cudaError_t launch_scan_u32(const uint32_t* in, uint32_t* out, long long n, void* tmp, cudaStream_t st) {
-    long long nt = (n + kTile - 1) / kTile;
-    uint32_t* sums = (uint32_t*)tmp;
-    if (nt == 0) {
-        cudaMemsetAsync(out, 0, sizeof(uint32_t), st);
-        return cudaGetLastError();
-    }
-    k_tile_sums<<<(unsigned)nt, kScanThreads, 0, st>>>(in, n, sums);
-    k_scan_sums<<<1, kScanThreads, 0, st>>>(sums, nt);
-    k_tile_scan<<<(unsigned)nt, kScanThreads, 0, st>>>(in, out, n, sums, nt);
-    count_launch(3);
-    return cudaGetLastError();
+    return scan<uint32_t>(in, out, nullptr, n, tmp, st);
+}
+
+cudaError_t launch_scan_pairs(const uint32_t* in, uint32_t* out, uint32_t* pairs, long long n, void* tmp,
+                              cudaStream_t st) {
+    return scan<unsigned long long>(in, out, pairs, n, tmp, st);
 }
 
 }  // namespace ariel

@@ -91,6 +91,7 @@ struct ariel_sim {
     long long np = 0, nc = 0, nf = 0;
     bool any_solid = false;
     bool inited = false;
+    bool pairs_stale = false;  // the last sort queued was the resampler's
     cudaStream_t stream = nullptr;
     bool own_stream = true;
     cudaMemPool_t pool = nullptr;  // set: every buffer comes from this stream-ordered pool

@@ -30,6 +30,10 @@ struct DevState {
     float4* svel4;
     float4* gpos4;    // slot -> P2G record: clamped grid position and mass (FLUID), far away
                       // for other particles so that they fall outside every face's radius
+    // the slots' positions and masses as pairs inside a cell, for the density's packed arithmetic:
+    // (x0 x1 y0 y1), (z0 z1 m0 m1); the second of a cell's odd last particle is far away, mass 0
+    uint32_t* pstart;  // cell -> first pair (nc+1)
+    float4* spair;
     float* dens;      // slot -> density
     // static solid particles binned by cell (positions never change)
     uint32_t* solid_start;  // nc+1
@@ -56,6 +60,8 @@ struct DevState {
 // Launchers (each returns cudaGetLastError()).
 cudaError_t launch_begin(const DevState& S, cudaStream_t st);
 cudaError_t launch_sort(const DevState& S, void* scan_tmp, cudaStream_t st);
+// the density's pair records when the last sort was the resampler's, which leaves them out
+cudaError_t launch_make_pairs(const DevState& S, void* scan_tmp, cudaStream_t st);
 cudaError_t launch_density(const DevState& S, cudaStream_t st);
 cudaError_t launch_forces(const DevState& S, cudaStream_t st);
 // faces: faces per thread (1, 2, 4), or 0 to choose by the number of faces
@@ -82,6 +88,11 @@ cudaError_t launch_pack_w(const float4* pos4, const float4* vel4, float* mass, i
 // scan_tmp_bytes(n) bytes.
 size_t scan_tmp_bytes(long long n);
 cudaError_t launch_scan_u32(const uint32_t* in, uint32_t* out, long long n, void* tmp, cudaStream_t st);
+// The same and, into pairs[0..n], the exclusive scan of the pairs (v + 1) / 2 that hold each v.
+cudaError_t launch_scan_pairs(const uint32_t* in, uint32_t* out, uint32_t* pairs, long long n, void* tmp,
+                              cudaStream_t st);
+// Most pairs of np particles in nc cells.
+inline long long pair_bound(long long np, long long nc) { return (np + (np < nc ? np : nc) + 1) / 2; }
 
 // Kernel-launch accounting (one increment per launched kernel).
 void count_launch(int n = 1);

@@ -1,0 +1,52 @@
+"""The density over pair records (csrc/particles.cu, k_density) bit for bit against the oracle:
+cells of few and odd numbers of particles up to the walls, solid particles among them, grids with
+and without a power-of-two kernel radius, and a radius far out of range; and the records rebuilt
+where the last sort was the resampler's, which leaves them out."""
+import numpy as np
+import pytest
+
+from ariel_b200 import _abi as A
+from ariel_b200.flipsim import Batch
+
+from helpers import assert_bits, dambreak, params
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,count,density", [(2, 1, 0.5), (2, 9, 0.5), (5, 2, 0.5), (16, 3000, 0.5), (31, 20001, 0.5),
+                                             (33, 40000, 0.3), (16, 500, 1e12), (12, 400, 1e-12)])
+def test_density_bits(n, count, density):
+    from oracle.pyoracle import RefSim
+    rng = np.random.default_rng(n + count)
+    desc = A.scene_dambreak(n, density=density)
+    prm = params()
+    pos = rng.random((count, 3)).astype(np.float32)
+    pos[rng.random(count) < 0.3] *= np.float32(0.2)  # crowded corner
+    pos[: count // 20] = np.round(pos[: count // 20])  # on the walls and in the corners
+    vel = np.zeros((count, 3), np.float32)
+    typ = np.where(rng.random(count) < 0.1, A.SOLID, A.FLUID).astype(np.int32)
+    mass = np.where(typ == A.SOLID, 10.0, 1.0 + rng.random(count)).astype(np.float32)
+    got = []
+    for make in (lambda: Batch([desc], prm), lambda: RefSim(desc, prm)):
+        s = make()
+        s.set_particles(pos, vel, mass, typ)
+        s.stage(A.STAGE_SORT)
+        s.stage(A.STAGE_DENSITY)
+        got.append(s.get_particles()["density"])
+        s.close()
+    assert_bits("density", got[0], got[1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("graph", [0, 1])
+def test_density_after_the_resamplers_sort(graph):
+    # no resampling: the step's last sort leaves every particle where a fresh sort finds it
+    b = Batch([dambreak(20), dambreak(13, seed=3)], params(graph=graph, resample_every=0))
+    b.init()
+    b.step(3)
+    b.stage(A.STAGE_DENSITY)
+    stale = [b.get_particles(s)["density"] for s in range(2)]
+    b.stage(A.STAGE_SORT)
+    b.stage(A.STAGE_DENSITY)
+    for s in range(2):
+        assert_bits("scene %d" % s, b.get_particles(s)["density"], stale[s])
+    b.close()
