@@ -35,6 +35,7 @@ struct FaceIdx {
 
 // ------------------------------------------------------------------------------------------
 __global__ void k_classify(DevState S) {
+    kernel_begin();
     SCENE_PREFIX(S.c_pref);
     long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= S.nc) return;
@@ -63,7 +64,7 @@ __global__ void k_classify(DevState S) {
 }
 
 // ------------------------------------------------------------------------------------------
-__device__ __forceinline__ float check_wall(const uint8_t* __restrict__ A, long long c) {
+__device__ __forceinline__ float check_wall(const uint8_t* A, long long c) {
     return A[c] == ARIEL_SOLID ? 1.0f : -1.0f;
 }
 
@@ -90,6 +91,7 @@ __device__ __forceinline__ void for_cells(const DevState& S, const long long* pr
 }
 
 __global__ void k_boundary_div(DevState S) {
+    kernel_begin();
     SCENE_PREFIX(S.c_pref);
     for_cells(S, pref_s, [&](long long c, const SceneDev& D, int i, int j, int k) {
         const int n = D.n;
@@ -174,6 +176,7 @@ __device__ __forceinline__ void for_faces(const DevState& S, const long long* pr
 }
 
 __global__ void k_gradient(DevState S) {
+    kernel_begin();
     SCENE_PREFIX(S.f_pref);
     for_faces(S, pref_s, [&](long long g, const SceneDev& D, int axis, int i, int j, int k) {
         const int n = D.n;
@@ -203,6 +206,7 @@ __global__ void k_gradient(DevState S) {
 
 // ------------------------------------------------------------------------------------------
 __global__ void k_extrapolate(DevState S) {
+    kernel_begin();
     SCENE_PREFIX(S.f_pref);
     for_faces(S, pref_s, [&](long long g, const SceneDev& D, int axis, int i, int j, int k) {
         const int n = D.n;
@@ -254,28 +258,28 @@ __global__ void k_extrapolate(DevState S) {
 cudaError_t launch_classify(const DevState& S, int init_density, cudaStream_t st) {
     (void)init_density;
     if (S.nc == 0) return cudaSuccess;
-    k_classify<<<grid_for(S.nc), kBlock, 0, st>>>(S);
+    launch_k(k_classify, grid_for(S.nc), kBlock, st, S);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_boundary_div(const DevState& S, cudaStream_t st) {
     if (S.nc == 0) return cudaSuccess;
-    k_boundary_div<<<grid_for((S.nc + kCellsPerThread - 1) / kCellsPerThread), kBlock, 0, st>>>(S);
+    launch_k(k_boundary_div, grid_for((S.nc + kCellsPerThread - 1) / kCellsPerThread), kBlock, st, S);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_gradient(const DevState& S, cudaStream_t st) {
     if (S.nf == 0) return cudaSuccess;
-    k_gradient<<<grid_for((S.nf + kFacesPerThread - 1) / kFacesPerThread), kBlock, 0, st>>>(S);
+    launch_k(k_gradient, grid_for((S.nf + kFacesPerThread - 1) / kFacesPerThread), kBlock, st, S);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_extrapolate(const DevState& S, cudaStream_t st) {
     if (S.nf == 0) return cudaSuccess;
-    k_extrapolate<<<grid_for((S.nf + kFacesPerThread - 1) / kFacesPerThread), kBlock, 0, st>>>(S);
+    launch_k(k_extrapolate, grid_for((S.nf + kFacesPerThread - 1) / kFacesPerThread), kBlock, st, S);
     count_launch();
     return cudaGetLastError();
 }

@@ -230,7 +230,7 @@ long long layout_bytes(const Layout& L) {
     add(nf, 4);      // u
     add(nf, 4);      // pu
     add(1, 4);       // dev_error
-    add((long long)scan_tmp_bytes(nc), 1);
+    add((long long)scan_tmp_bytes(nc) + 16, 1);
     if (L.any_reseed) {
         add(nc, 4);      // reseed: excess
         add(nc + 1, 4);  // its scan
@@ -592,7 +592,7 @@ ariel_status build_state(ariel_sim* s, std::vector<HostParticles>& hp, const ari
     ARIEL_TRY(dalloc(s, &S.u, nf));
     ARIEL_TRY(dalloc(s, &S.pu, nf));
     ARIEL_TRY(dalloc(s, &S.dev_error, 1));
-    size_t st_bytes = scan_tmp_bytes(nc);
+    size_t st_bytes = scan_tmp_bytes(nc) + 16;  // with the sort's counter of crowded cells
     char* tmp = nullptr;
     ARIEL_TRY(dalloc(s, &tmp, st_bytes));
     s->scan_tmp = tmp;

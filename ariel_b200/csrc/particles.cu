@@ -125,11 +125,13 @@ __device__ void solid_constraints(const SceneDev& D, float3& p, float3& u, float
 // BEGIN: frame++, AdjustParticlesStuckInSolids (flip.cpp:130-181), StoreTemp (flip.cpp:79-90)
 // ------------------------------------------------------------------------------------------
 __global__ void k_frame_inc(SceneDev* scenes, int k) {
+    kernel_begin();
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s < k) scenes[s].frame += 1;
 }
 
 __global__ void k_begin_solids(DevState S) {
+    kernel_begin();
     SCENE_PREFIX(S.p_pref);
     long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= S.np) return;
@@ -170,7 +172,15 @@ __global__ void k_begin_solids(DevState S) {
 // ------------------------------------------------------------------------------------------
 // Sort-by-cell (replaces ParticleGrid::Sort, particlegrid.cpp:140-172)
 // ------------------------------------------------------------------------------------------
+__global__ void k_sort_zero(DevState S, uint32_t* nbig) {
+    kernel_begin();
+    const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (c < S.nc) S.count[c] = 0u;
+    if (c == 0) *nbig = 0u;
+}
+
 __global__ void k_sort_key(DevState S) {
+    kernel_begin();
     SCENE_PREFIX(S.p_pref);
     long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= S.np) return;
@@ -184,6 +194,7 @@ __global__ void k_sort_key(DevState S) {
 }
 
 __global__ void k_sort_scatter(DevState S) {
+    kernel_begin();
     long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= S.np) return;
     uint32_t c = S.key[g];
@@ -195,6 +206,7 @@ __global__ void k_sort_scatter(DevState S) {
 // array, free once the scatter has run; `nbig` counts them) for k_sort_big.
 constexpr int kSortRegs = 16;
 __global__ void k_sort_cells(DevState S, uint32_t* nbig) {
+    kernel_begin();
     long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= S.nc) return;
     uint32_t a = S.start[c], b = S.start[c + 1];
@@ -233,6 +245,7 @@ constexpr int kBigCell = 1024;
 constexpr int kBigWarps = 8;
 constexpr int kSortBigBlocks = 296;  // a grid-stride loop over the listed cells
 __global__ void __launch_bounds__(32 * kBigWarps) k_sort_big(DevState S, const uint32_t* nbig) {
+    kernel_begin();
     __shared__ uint32_t buf[kBigWarps][kBigCell];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t count = *nbig;
@@ -294,6 +307,7 @@ __device__ __forceinline__ void write_pairs(const DevState& S, const SceneDev& D
 
 template <bool PAIRS>
 __global__ void k_sort_permute(DevState S) {
+    kernel_begin();
     SCENE_PREFIX(S.p_pref);
     long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const bool in = s < S.np;
@@ -323,6 +337,7 @@ __global__ void k_sort_permute(DevState S) {
 
 // The pair records of slots sorted without them (the resampler's Sort).
 __global__ void k_make_pairs(DevState S) {
+    kernel_begin();
     SCENE_PREFIX(S.p_pref);
     const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const bool in = s < S.np;
@@ -395,7 +410,7 @@ __device__ __forceinline__ float2 smooth_pair(float2 x, float2 y, float2 z, floa
 }
 
 template <int DIV>
-__device__ __forceinline__ void density_run(const float4* __restrict__ sp, uint32_t a, uint32_t b, const float2 (&n0)[3],
+__device__ __forceinline__ void density_run(const float4* sp, uint32_t a, uint32_t b, const float2 (&n0)[3],
                                             const float2 (&n1)[3], float hh, float ninv, float2 nzero, float& sum0,
                                             float& sum1) {
 #pragma unroll 2
@@ -414,6 +429,7 @@ __device__ __forceinline__ void density_run(const float4* __restrict__ sp, uint3
 
 constexpr int kDensityBlock = 256;
 __global__ void __launch_bounds__(kDensityBlock, 4) k_density(DevState S, float neg_zero) {
+    kernel_begin();
     __shared__ long long pref_s[kMaxScenes + 1];  // pair begins of the scenes
     for (int i = threadIdx.x; i <= S.k; i += blockDim.x) pref_s[i] = S.pstart[S.c_pref[i]];
     __syncthreads();
@@ -448,11 +464,13 @@ __global__ void __launch_bounds__(kDensityBlock, 4) k_density(DevState S, float 
 }
 
 __global__ void k_fill_dens(DevState S, float v) {
+    kernel_begin();
     long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (s < S.np) S.dens[s] = v;
 }
 
 __global__ void k_scatter_density(DevState S, float* out) {
+    kernel_begin();
     long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (s < S.np) out[S.sid[s]] = S.dens[s];
 }
@@ -461,6 +479,7 @@ __global__ void k_scatter_density(DevState S, float* out) {
 // FlipSim::ApplyExternalForces (flip.cpp:682-695): on the slot copy and the id-order state.
 // ------------------------------------------------------------------------------------------
 __global__ void k_forces(DevState S) {
+    kernel_begin();
     SCENE_PREFIX(S.p_pref);
     long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= S.np) return;
@@ -501,7 +520,7 @@ __device__ __forceinline__ float face_offset_z(int axis, int k) { return axis ==
 
 template <int F>
 __device__ __forceinline__ void p2g_row(const DevState& S, const SceneDev& D, int axis, int i, int j, int k, int nk,
-                                        float* __restrict__ out) {
+                                        float* out) {
     const int n = D.n;
     // face centre (x, y shared by the row) and the union of the GetWallNeighbors blocks
     // [index - nn, index + nn - 1] of faces k .. k + nk - 1
@@ -531,7 +550,7 @@ __device__ __forceinline__ void p2g_row(const DevState& S, const SceneDev& D, in
 #pragma unroll
     for (int f = 0; f < F; ++f) fz[f] = face_offset_z(axis, k + f);
     const float2 nfxy = make_float2(-fx, -fy);
-    const float* __restrict__ vel = reinterpret_cast<const float*>(S.svel4) + axis;
+    const float* vel = reinterpret_cast<const float*>(S.svel4) + axis;
     const float maxd_m1 = D.maxd - 1.0f;
     float sumw[F], sumu[F];
 #pragma unroll
@@ -602,6 +621,7 @@ __device__ __forceinline__ void p2g_row(const DevState& S, const SceneDev& D, in
 // faster; six blocks, at 40 registers with spills, are slower).
 template <int F>
 __global__ void __launch_bounds__(kBlock, 5) k_p2g(DevState S, long long third) {
+    kernel_begin();
     SCENE_PREFIX(S.f_pref);
     const long long grp = (long long)(blockIdx.x % 3) * third + (long long)(blockIdx.x / 3) * blockDim.x + threadIdx.x;
     long long g = grp * F;
@@ -622,7 +642,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_p2g(DevState S, long long third) 
 // ------------------------------------------------------------------------------------------
 // Interpolate / InterpolateVelocity (particlegridoperations.inl:106-133)
 // ------------------------------------------------------------------------------------------
-__device__ __forceinline__ float interp1(const float* __restrict__ q, int ey, int ez, float px, float py, float pz,
+__device__ __forceinline__ float interp1(const float* q, int ey, int ez, float px, float py, float pz,
                                          float nx, float ny, float nz) {
     float x = gmax(0.0f, gmin(nx, px));
     float y = gmax(0.0f, gmin(ny, py));
@@ -639,7 +659,7 @@ __device__ __forceinline__ float interp1(const float* __restrict__ q, int ey, in
     return (fk1 - z) * (term1 + term2) + (z - k) * (term3 + term4);
 }
 
-__device__ __forceinline__ float3 interp_vel(const float* __restrict__ faces, int n, float3 p) {
+__device__ __forceinline__ float3 interp_vel(const float* faces, int n, float3 p) {
     const long long per = (long long)n * n * (n + 1);
     const float X = (float)n;
     float3 u;
@@ -654,6 +674,7 @@ __device__ __forceinline__ float3 interp_vel(const float* __restrict__ faces, in
 // CheckParticleSolidConstraints (flip.cpp:183-227), one thread per particle (id order).
 // ------------------------------------------------------------------------------------------
 __global__ void k_g2p_advect(DevState S) {
+    kernel_begin();
     SCENE_PREFIX(S.p_pref);
     long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= S.np) return;
@@ -776,6 +797,7 @@ __device__ __forceinline__ void column_slots(const DevState& S, const SceneDev& 
 // exact arithmetic.  Neighbours outside the radius contribute exactly nothing.
 // Five blocks per SM (51 registers, a 12-byte spill): 1-2% faster than four.
 __global__ void __launch_bounds__(kBlock, 5) k_resample_spring(DevState S) {
+    kernel_begin();
     SCENE_PREFIX(S.p_pref);
     __shared__ uint32_t lst[kResList][kBlock];
     const int me = threadIdx.x;
@@ -871,6 +893,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_resample_spring(DevState S) {
 }
 
 __global__ void __launch_bounds__(kBlock, 4) k_resample_velocity(DevState S) {
+    kernel_begin();
     SCENE_PREFIX(S.p_pref);
     __shared__ uint32_t lst[kResList][kBlock];
     const int me = threadIdx.x;
@@ -973,6 +996,7 @@ __device__ __forceinline__ bool reseed_frame(const SceneDev& D) {
 }
 
 __global__ void k_reseed_count(DevState S) {
+    kernel_begin();
     SCENE_PREFIX(S.c_pref);
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= S.nc) return;
@@ -1003,7 +1027,7 @@ __global__ void k_reseed_count(DevState S) {
 // One thread per given particle (grid-stride over the scan's total, so a crowded cell's
 // particles spread over many threads): the giving cell and the receiving cell are found by
 // binary search over the two scans.
-__device__ __forceinline__ long long last_at_or_below(const uint32_t* __restrict__ scan, long long lo, long long hi,
+__device__ __forceinline__ long long last_at_or_below(const uint32_t* scan, long long lo, long long hi,
                                                       uint32_t v) {
     // the largest q in [lo, hi] with scan[q] <= v (scan does not decrease; scan[lo] <= v)
     while (lo < hi) {
@@ -1019,6 +1043,7 @@ __device__ __forceinline__ long long last_at_or_below(const uint32_t* __restrict
 constexpr int kReseedBlocks = 4 * 148;  // four blocks on each of a B200's SMs
 
 __global__ void k_reseed_move(DevState S) {
+    kernel_begin();
     SCENE_PREFIX(S.c_pref);
     const uint32_t total = S.rs_escan[S.nc];
     for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < total; x += gridDim.x * blockDim.x) {
@@ -1051,8 +1076,9 @@ __global__ void k_reseed_move(DevState S) {
     }
 }
 
-__global__ void k_unpack_state(float4* pos4, float4* vel4, const float* __restrict__ pos,
-                               const float* __restrict__ vel, long long n, int* err) {
+__global__ void k_unpack_state(float4* pos4, float4* vel4, const float* pos,
+                               const float* vel, long long n, int* err) {
+    kernel_begin();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float4 p = pos4[i], v = vel4[i];
@@ -1068,8 +1094,9 @@ __global__ void k_unpack_state(float4* pos4, float4* vel4, const float* __restri
     vel4[i] = v;
 }
 
-__global__ void k_pack_state(const float4* __restrict__ pos4, const float4* __restrict__ vel4, float* pos, float* vel,
+__global__ void k_pack_state(const float4* pos4, const float4* vel4, float* pos, float* vel,
                              long long n) {
+    kernel_begin();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float4 p = pos4[i], v = vel4[i];
@@ -1081,8 +1108,9 @@ __global__ void k_pack_state(const float4* __restrict__ pos4, const float4* __re
     vel[3 * i + 2] = v.z;
 }
 
-__global__ void k_pack_w(const float4* __restrict__ pos4, const float4* __restrict__ vel4, float* mass, int32_t* type,
+__global__ void k_pack_w(const float4* pos4, const float4* vel4, float* mass, int32_t* type,
                          long long n) {
+    kernel_begin();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     mass[i] = pos4[i].w;
@@ -1094,7 +1122,7 @@ __global__ void k_pack_w(const float4* __restrict__ pos4, const float4* __restri
 cudaError_t launch_pack_w(const float4* pos4, const float4* vel4, float* mass, int32_t* type, long long n,
                           cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    k_pack_w<<<grid_for(n), kBlock, 0, st>>>(pos4, vel4, mass, type, n);
+    launch_k(k_pack_w, grid_for(n), kBlock, st, pos4, vel4, mass, type, n);
     count_launch();
     return cudaGetLastError();
 }
@@ -1102,7 +1130,7 @@ cudaError_t launch_pack_w(const float4* pos4, const float4* vel4, float* mass, i
 cudaError_t launch_unpack_state(float4* pos4, float4* vel4, const float* pos, const float* vel, long long n,
                                 int* err, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    k_unpack_state<<<grid_for(n), kBlock, 0, st>>>(pos4, vel4, pos, vel, n, err);
+    launch_k(k_unpack_state, grid_for(n), kBlock, st, pos4, vel4, pos, vel, n, err);
     count_launch();
     return cudaGetLastError();
 }
@@ -1110,7 +1138,7 @@ cudaError_t launch_unpack_state(float4* pos4, float4* vel4, const float* pos, co
 cudaError_t launch_pack_state(const float4* pos4, const float4* vel4, float* pos, float* vel, long long n,
                               cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    k_pack_state<<<grid_for(n), kBlock, 0, st>>>(pos4, vel4, pos, vel, n);
+    launch_k(k_pack_state, grid_for(n), kBlock, st, pos4, vel4, pos, vel, n);
     count_launch();
     return cudaGetLastError();
 }
@@ -1119,35 +1147,35 @@ cudaError_t launch_pack_state(const float4* pos4, const float4* vel4, float* pos
 // launchers
 // ------------------------------------------------------------------------------------------
 cudaError_t launch_begin(const DevState& S, cudaStream_t st) {
-    k_frame_inc<<<grid_for(S.k), kBlock, 0, st>>>(const_cast<SceneDev*>(S.scenes), S.k);
+    launch_k(k_frame_inc, grid_for(S.k), kBlock, st, const_cast<SceneDev*>(S.scenes), S.k);
     count_launch();
     if (S.any_solid && S.np > 0) {
-        k_begin_solids<<<grid_for(S.np), kBlock, 0, st>>>(S);
+        launch_k(k_begin_solids, grid_for(S.np), kBlock, st, S);
         count_launch();
     }
     return cudaGetLastError();
 }
 
 static cudaError_t sort_core(const DevState& S, void* scan_tmp, bool pairs, cudaStream_t st) {
-    cudaMemsetAsync(S.count, 0, sizeof(uint32_t) * (size_t)S.nc, st);
+    // a word behind the scan's scratch counts the cells for k_sort_big
+    uint32_t* nbig = reinterpret_cast<uint32_t*>(static_cast<char*>(scan_tmp) + scan_tmp_bytes(S.nc));
+    launch_k(k_sort_zero, grid_for(S.nc), kBlock, st, S, nbig);
+    count_launch();
     if (S.np > 0) {
-        k_sort_key<<<grid_for(S.np), kBlock, 0, st>>>(S);
+        launch_k(k_sort_key, grid_for(S.np), kBlock, st, S);
         count_launch();
     }
     cudaError_t e = pairs ? launch_scan_pairs(S.count, S.start, S.pstart, S.nc, scan_tmp, st)
                           : launch_scan_u32(S.count, S.start, S.nc, scan_tmp, st);
     if (e != cudaSuccess) return e;
     if (S.np > 0) {
-        // the scan's scratch is free again: its first word counts the cells for k_sort_big
-        uint32_t* nbig = reinterpret_cast<uint32_t*>(scan_tmp);
-        k_sort_scatter<<<grid_for(S.np), kBlock, 0, st>>>(S);
-        cudaMemsetAsync(nbig, 0, sizeof(uint32_t), st);
-        k_sort_cells<<<grid_for(S.nc), kBlock, 0, st>>>(S, nbig);
-        k_sort_big<<<kSortBigBlocks, 32 * kBigWarps, 0, st>>>(S, nbig);
+        launch_k(k_sort_scatter, grid_for(S.np), kBlock, st, S);
+        launch_k(k_sort_cells, grid_for(S.nc), kBlock, st, S, nbig);
+        launch_k(k_sort_big, kSortBigBlocks, 32 * kBigWarps, st, S, nbig);
         if (pairs)
-            k_sort_permute<true><<<grid_for(S.np), kBlock, 0, st>>>(S);
+            launch_k(k_sort_permute<true>, grid_for(S.np), kBlock, st, S);
         else
-            k_sort_permute<false><<<grid_for(S.np), kBlock, 0, st>>>(S);
+            launch_k(k_sort_permute<false>, grid_for(S.np), kBlock, st, S);
         count_launch(4);
     }
     return cudaGetLastError();
@@ -1159,35 +1187,35 @@ cudaError_t launch_make_pairs(const DevState& S, void* scan_tmp, cudaStream_t st
     if (S.np == 0) return cudaSuccess;
     cudaError_t e = launch_scan_pairs(S.count, S.start, S.pstart, S.nc, scan_tmp, st);
     if (e != cudaSuccess) return e;
-    k_make_pairs<<<grid_for(S.np), kBlock, 0, st>>>(S);
+    launch_k(k_make_pairs, grid_for(S.np), kBlock, st, S);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_density(const DevState& S, cudaStream_t st) {
     if (S.np == 0) return cudaSuccess;
-    k_density<<<grid_for(pair_bound(S.np, S.nc), kDensityBlock), kDensityBlock, 0, st>>>(S, -0.0f);
+    launch_k(k_density, grid_for(pair_bound(S.np, S.nc), kDensityBlock), kDensityBlock, st, S, -0.0f);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_fill_dens(const DevState& S, float value, cudaStream_t st) {
     if (S.np == 0) return cudaSuccess;
-    k_fill_dens<<<grid_for(S.np), kBlock, 0, st>>>(S, value);
+    launch_k(k_fill_dens, grid_for(S.np), kBlock, st, S, value);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_scatter_density(const DevState& S, float* out, cudaStream_t st) {
     if (S.np == 0) return cudaSuccess;
-    k_scatter_density<<<grid_for(S.np), kBlock, 0, st>>>(S, out);
+    launch_k(k_scatter_density, grid_for(S.np), kBlock, st, S, out);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_forces(const DevState& S, cudaStream_t st) {
     if (S.np == 0) return cudaSuccess;
-    k_forces<<<grid_for(S.np), kBlock, 0, st>>>(S);
+    launch_k(k_forces, grid_for(S.np), kBlock, st, S);
     count_launch();
     return cudaGetLastError();
 }
@@ -1202,18 +1230,18 @@ cudaError_t launch_p2g(const DevState& S, int faces, cudaStream_t st) {
     const long long third_blocks = (groups + 3LL * kBlock - 1) / (3LL * kBlock);
     const unsigned blocks = (unsigned)(3 * third_blocks);
     if (F == 4)
-        k_p2g<4><<<blocks, kBlock, 0, st>>>(S, third_blocks * kBlock);
+        launch_k(k_p2g<4>, blocks, kBlock, st, S, third_blocks * kBlock);
     else if (F == 2)
-        k_p2g<2><<<blocks, kBlock, 0, st>>>(S, third_blocks * kBlock);
+        launch_k(k_p2g<2>, blocks, kBlock, st, S, third_blocks * kBlock);
     else
-        k_p2g<1><<<blocks, kBlock, 0, st>>>(S, third_blocks * kBlock);
+        launch_k(k_p2g<1>, blocks, kBlock, st, S, third_blocks * kBlock);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_g2p_advect(const DevState& S, cudaStream_t st) {
     if (S.np == 0) return cudaSuccess;
-    k_g2p_advect<<<grid_for(S.np), kBlock, 0, st>>>(S);
+    launch_k(k_g2p_advect, grid_for(S.np), kBlock, st, S);
     count_launch();
     return cudaGetLastError();
 }
@@ -1225,18 +1253,18 @@ cudaError_t launch_resample(const DevState& S, void* scan_tmp, cudaStream_t st) 
     cudaError_t e = sort_core(S, scan_tmp, false, st);
     if (e != cudaSuccess) return e;
     if (S.np == 0) return cudaSuccess;
-    k_resample_spring<<<grid_for(S.np), kBlock, 0, st>>>(S);
-    k_resample_velocity<<<grid_for(S.np), kBlock, 0, st>>>(S);
+    launch_k(k_resample_spring, grid_for(S.np), kBlock, st, S);
+    launch_k(k_resample_velocity, grid_for(S.np), kBlock, st, S);
     count_launch(2);
     if (S.any_reseed) {
         // the kernels return at once on frames without reseeding; the scans stay (cheap)
-        k_reseed_count<<<grid_for(S.nc), kBlock, 0, st>>>(S);
+        launch_k(k_reseed_count, grid_for(S.nc), kBlock, st, S);
         count_launch();
         e = launch_scan_u32(S.rs_excess, S.rs_escan, S.nc, scan_tmp, st);
         if (e != cudaSuccess) return e;
         e = launch_scan_u32(S.rs_deficit, S.rs_dscan, S.nc, scan_tmp, st);
         if (e != cudaSuccess) return e;
-        k_reseed_move<<<kReseedBlocks, kBlock, 0, st>>>(S);
+        launch_k(k_reseed_move, kReseedBlocks, kBlock, st, S);
         count_launch();
     }
     return cudaGetLastError();

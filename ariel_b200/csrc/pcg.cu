@@ -177,7 +177,20 @@ __device__ __forceinline__ int list_order(int n, int i, int j, int k) {
     return (i0 * n + j0 * bi) * n + k0 * bi * bj + ((i - i0) * bj + (j - j0)) * bk + (k - k0);
 }
 
+// Clears the solver's records, control words and brick flags.
+__global__ void k_pcg_zero(PcgArgs A) {
+    kernel_begin();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < A.S.k) A.sc[i] = PcgScene{};
+    if (i < A.nbricks) A.bflag[i] = 0u;
+    if (i == 0) {
+        *A.ctl = PcgCtl{};
+        *A.bar = Barrier{};
+    }
+}
+
 __global__ void k_prep_cells(PcgArgs A, uint32_t* pred) {
+    kernel_begin();
     const DevState& S = A.S;
     __shared__ long long pref_s[kMaxScenes + 1];
     load_prefix<kMaxScenes>(pref_s, S.c_pref, S.k);
@@ -248,41 +261,12 @@ __global__ void k_prep_cells(PcgArgs A, uint32_t* pred) {
     if (one) atomicAdd(&A.sc[s].ones, 1);
 }
 
-// FLUID list, plus one 16-byte record per entry holding everything the solve needs about the
-// cell besides its vectors: index, neighbour mask and ADiag (fp32 bits for the fp32 modes, fp64
-// bits otherwise), so that a single load starts a cell's update.
-__global__ void k_fl_write(PcgArgs A, const uint32_t* scan) {
-    const DevState& S = A.S;
-    __shared__ long long pref_s[kMaxScenes + 1];
-    load_prefix<kMaxScenes>(pref_s, S.c_pref, S.k);
-    long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= S.nc) return;
-    if (S.flags[c] != ARIEL_FLUID) return;
-    const SceneDev& D = S.scenes[find_scene(pref_s, S.k, c)];
-    int i, j, k;
-    cell_ijk(D, c - D.c_begin, i, j, k);
-    const uint32_t t = scan[D.c_begin + list_order(D.n, i, j, k)];
-    const_cast<uint32_t*>(A.fl)[t] = (uint32_t)c;
-    uint4 r;
-    r.x = (uint32_t)c;
-    r.y = (uint32_t)A.mask[c];
-    if (A.mode == kFp64) {
-        const unsigned long long b = (unsigned long long)__double_as_longlong(A.diag[c]);
-        r.z = (uint32_t)b;
-        r.w = (uint32_t)(b >> 32);
-    } else {
-        r.z = __float_as_uint((float)A.diag[c]);
-        r.w = 0u;
-    }
-    A.rec[t] = r;
-}
-
 // Per-scene tables of the solve, one block.  A resident scene gets a range of block positions
 // inside one group of A.res_blocks; the scenes of a class take as few chunks per block as put them
 // all in one group, and are packed into groups by falling size (first fit).  The others keep their
 // chunks in ch_pref for the streaming kernel.
-constexpr int kTableThreads = 256;
-__global__ void __launch_bounds__(kTableThreads) k_pcg_tables(PcgArgs A, const uint32_t* scan) {
+constexpr int kTableThreads = kBlock;
+__device__ void pcg_tables(const PcgArgs& A, const uint32_t* scan) {
     const int k = A.S.k, G = A.res_blocks;
     __shared__ int nch_s[kMaxScenes], csz_s[kMaxScenes], order_s[kResMaxScenes], fill_s[kResMaxScenes];
     __shared__ int need_s[kResClasses][4];  // positions of a class at 1, 2, 4, 8 chunks per block
@@ -355,6 +339,41 @@ __global__ void __launch_bounds__(kTableThreads) k_pcg_tables(PcgArgs A, const u
     A.ctl->all_inner_done = 0;
     A.ctl->any_ordered = any_ordered;
     A.ctl->nstream = nstream;
+}
+
+// FLUID list, plus one 16-byte record per entry holding everything the solve needs about the
+// cell besides its vectors: index, neighbour mask and ADiag (fp32 bits for the fp32 modes, fp64
+// bits otherwise), so that a single load starts a cell's update.
+__global__ void k_fl_write(PcgArgs A, const uint32_t* scan) {
+    kernel_begin();
+    // the first block makes the tables, which need nothing but the scan either
+    if (blockIdx.x == 0) {
+        pcg_tables(A, scan);
+        return;
+    }
+    const DevState& S = A.S;
+    __shared__ long long pref_s[kMaxScenes + 1];
+    load_prefix<kMaxScenes>(pref_s, S.c_pref, S.k);
+    long long c = (long long)(blockIdx.x - 1) * blockDim.x + threadIdx.x;
+    if (c >= S.nc) return;
+    if (S.flags[c] != ARIEL_FLUID) return;
+    const SceneDev& D = S.scenes[find_scene(pref_s, S.k, c)];
+    int i, j, k;
+    cell_ijk(D, c - D.c_begin, i, j, k);
+    const uint32_t t = scan[D.c_begin + list_order(D.n, i, j, k)];
+    const_cast<uint32_t*>(A.fl)[t] = (uint32_t)c;
+    uint4 r;
+    r.x = (uint32_t)c;
+    r.y = (uint32_t)A.mask[c];
+    if (A.mode == kFp64) {
+        const unsigned long long b = (unsigned long long)__double_as_longlong(A.diag[c]);
+        r.z = (uint32_t)b;
+        r.w = (uint32_t)(b >> 32);
+    } else {
+        r.z = __float_as_uint((float)A.diag[c]);
+        r.w = 0u;
+    }
+    A.rec[t] = r;
 }
 
 // Data written by other blocks is read only after a grid barrier (whose acquire makes ordinary
@@ -1349,21 +1368,15 @@ __global__ void k_barrier_selftest(Barrier* bar, int* err, unsigned long long tm
 
 cudaError_t launch_pcg_prepare(const PcgArgs& A, uint32_t* pred, uint32_t* scan, void* scan_tmp, cudaStream_t st) {
     const DevState& S = A.S;
-    cudaMemsetAsync(A.sc, 0, sizeof(PcgScene) * (size_t)S.k, st);
-    cudaMemsetAsync(A.ctl, 0, sizeof(PcgCtl), st);
-    cudaMemsetAsync(A.bar, 0, sizeof(Barrier), st);
-    if (A.nbricks > 0) cudaMemsetAsync(A.bflag, 0, sizeof(unsigned) * (size_t)A.nbricks, st);
+    launch_k(k_pcg_zero, grid_for(std::max<long long>(A.nbricks, S.k)), kBlock, st, A);
+    count_launch();
     if (S.nc > 0) {
-        k_prep_cells<<<grid_for(S.nc), kBlock, 0, st>>>(A, pred);
+        launch_k(k_prep_cells, grid_for(S.nc), kBlock, st, A, pred);
         count_launch();
     }
     cudaError_t e = launch_scan_u32(pred, scan, S.nc, scan_tmp, st);
     if (e != cudaSuccess) return e;
-    if (S.nc > 0) {
-        k_fl_write<<<grid_for(S.nc), kBlock, 0, st>>>(A, scan);
-        count_launch();
-    }
-    k_pcg_tables<<<1, kTableThreads, 0, st>>>(A, scan);
+    launch_k(k_fl_write, 1 + grid_for(S.nc), kBlock, st, A, scan);
     count_launch();
     return cudaGetLastError();
 }

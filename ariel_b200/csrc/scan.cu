@@ -1,7 +1,7 @@
 // scan.cu -- exclusive prefix sum of uint32 counts (cell histograms, FLUID-cell compaction).
 //
-// Three passes over tiles of 4096 values: per-tile sums, one block scanning the tile sums,
-// per-tile scan plus offset.  Integer arithmetic, so the result does not depend on the order
+// Passes over tiles of 4096 values: per-tile sums, with many tiles one block scanning the tile
+// sums, per-tile scan plus offset.  Integer arithmetic, so the result does not depend on the order
 // in which blocks run.
 #include <atomic>
 
@@ -13,6 +13,7 @@ namespace {
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 16;
 constexpr int kTile = kScanThreads * kScanItems;
+constexpr long long kOwnPrefix = 1024;  // tiles (4 M values) up to which every block adds the earlier tiles' sums
 
 template <class T>
 __device__ __forceinline__ T warp_incl_scan(T v) {
@@ -61,7 +62,8 @@ __device__ __forceinline__ void put(uint32_t* out, uint32_t* pairs, long long i,
 }
 
 template <class T>
-__global__ void k_tile_sums(const uint32_t* __restrict__ in, long long n, T* __restrict__ sums) {
+__global__ void k_tile_sums(const uint32_t* in, long long n, T* sums) {
+    kernel_begin();
     long long base = (long long)blockIdx.x * kTile;
     T acc = 0;
 #pragma unroll
@@ -78,6 +80,7 @@ __global__ void k_tile_sums(const uint32_t* __restrict__ in, long long n, T* __r
 
 template <class T>
 __global__ void k_scan_sums(T* sums, long long nt) {
+    kernel_begin();
     __shared__ T carry_s;
     if (threadIdx.x == 0) carry_s = 0;
     __syncthreads();
@@ -95,9 +98,12 @@ __global__ void k_scan_sums(T* sums, long long nt) {
     if (threadIdx.x == 0) sums[nt] = carry_s;
 }
 
-template <class T>
-__global__ void k_tile_scan(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, uint32_t* __restrict__ pairs,
-                            long long n, const T* __restrict__ sums, long long nt) {
+// SUMMED: `sums` holds the exclusive prefixes of the tiles (k_scan_sums); else the tiles' own sums,
+// and each block adds those before it itself, which spares a launch while the tiles are few.
+template <class T, bool SUMMED>
+__global__ void k_tile_scan(const uint32_t* in, uint32_t* out, uint32_t* pairs,
+                            long long n, const T* sums, long long nt) {
+    kernel_begin();
     long long base = (long long)blockIdx.x * kTile + (long long)threadIdx.x * kScanItems;
     T vals[kScanItems];
     T acc = 0;
@@ -108,15 +114,24 @@ __global__ void k_tile_scan(const uint32_t* __restrict__ in, uint32_t* __restric
         if (i < n) widen(in[i], vals[it]);
         acc += vals[it];
     }
-    __shared__ T tot;
-    T ex = block_excl_scan(acc, &tot) + sums[blockIdx.x];
+    __shared__ T tot, before_s;
+    T before;
+    if (SUMMED) {
+        before = sums[blockIdx.x];
+    } else {
+        T b = 0;
+        for (long long i = threadIdx.x; i < (long long)blockIdx.x; i += kScanThreads) b += sums[i];
+        block_excl_scan(b, &before_s);
+        before = before_s;
+    }
+    T ex = block_excl_scan(acc, &tot) + before;
 #pragma unroll
     for (int it = 0; it < kScanItems; ++it) {
         long long i = base + it;
         if (i < n) put(out, pairs, i, ex);
         ex += vals[it];
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) put(out, pairs, n, sums[nt]);
+    if ((long long)blockIdx.x == nt - 1 && threadIdx.x == 0) put(out, pairs, n, before + tot);
 }
 
 template <class T>
@@ -128,10 +143,15 @@ cudaError_t scan(const uint32_t* in, uint32_t* out, uint32_t* pairs, long long n
         if (pairs) cudaMemsetAsync(pairs, 0, sizeof(uint32_t), st);
         return cudaGetLastError();
     }
-    k_tile_sums<T><<<(unsigned)nt, kScanThreads, 0, st>>>(in, n, sums);
-    k_scan_sums<T><<<1, kScanThreads, 0, st>>>(sums, nt);
-    k_tile_scan<T><<<(unsigned)nt, kScanThreads, 0, st>>>(in, out, pairs, n, sums, nt);
-    count_launch(3);
+    launch_k(k_tile_sums<T>, nt, kScanThreads, st, in, n, sums);
+    if (nt <= kOwnPrefix) {
+        launch_k(k_tile_scan<T, false>, nt, kScanThreads, st, in, out, pairs, n, sums, nt);
+        count_launch(2);
+    } else {
+        launch_k(k_scan_sums<T>, 1, kScanThreads, st, sums, nt);
+        launch_k(k_tile_scan<T, true>, nt, kScanThreads, st, in, out, pairs, n, sums, nt);
+        count_launch(3);
+    }
     return cudaGetLastError();
 }
 
