@@ -662,6 +662,7 @@ ariel_status build_state(ariel_sim* s, std::vector<HostParticles>& hp, const ari
     ARIEL_TRY(dalloc(s, &A.res, k));
     ARIEL_TRY(dalloc(s, &A.res_count, 32 * (size_t)k));
     A.flscan = s->flscan;
+    A.hlist = s->flpred;  // free once the list is written
     // bricks of the ordered sweeps: every scene's brick grid, listed by level I+J+K, then scene
     // and position (the order the sweeps take them in)
     sweep_brick(s->prm, A.bx, A.by, A.bz);
@@ -722,13 +723,21 @@ ariel_status build_state(ariel_sim* s, std::vector<HostParticles>& hp, const ari
     A.all_resident = A.res_blocks > 0;
     A.classes = 0;
     for (int i = 0; i < k; ++i) {
-        // over every FLUID count that the scene's grid allows
-        const long long n = s->descs[i].dim;
-        const int most = chunk_size(n * n * n);
-        for (int c = kChunkMin; c <= most; c += kChunkAlign) A.classes |= 1 << res_class(k, c);
-        if (chunk_bound(n * n * n) > std::min(kResMaxChunks, A.res_blocks * res_max_cpb(s->mode, k, most)))
+        // over the FLUID counts that the scene's grid allows: one per chunk size, and the largest
+        const long long n = s->descs[i].dim, most = n * n * n;
+        for (int c = kChunkMin; c <= chunk_size(most); c += kChunkAlign) {
+            const int m = (int)std::min(chunk_bound(most), kChunkTarget);
+            A.classes |= 1 << res_class(k, c, m);
+            const int cpb = res_max_cpb(s->mode, k, c, m);
+            if (m > A.res_blocks * cpb || !res_never_over(s->mode, c, cpb)) A.all_resident = 0;
+        }
+        if (chunk_bound(most) > kChunkTarget) {
+            A.classes |= 1 << kResBig;
             A.all_resident = 0;
+        }
     }
+    if (s->mode != kMixed) A.classes &= ~(1 << kResBig);
+    if (s->mode == kFp64 && k > 1) A.classes = A.all_resident = 0;
     cudaStream_t st = s->stream;
     // scene table and prefixes
     ARIEL_CUDA(cudaMemcpyAsync(s->d_scenes, s->sh.data(), sizeof(SceneDev) * k, cudaMemcpyHostToDevice, st));

@@ -167,11 +167,15 @@ struct VT<kFp64> {
 // ------------------------------------------------------------------------------------------
 // Preparation: per-cell operator data, order-free preconditioner, FLUID predicate.
 // ------------------------------------------------------------------------------------------
-// The FLUID list follows the cells brick by brick (8 x 8 x 32 cells, cut off at the far walls)
-// instead of the whole grid's (i, j, k) order: a chunk of consecutive entries is then a compact
-// piece of the liquid, with about 0.6 neighbours outside it per cell where a chunk of whole grid
-// rows has 2.1, and still runs of up to 32 consecutive cells along z.
-__device__ __forceinline__ int list_order(int n, int i, int j, int k) {
+// The fp32 modes' FLUID list follows the cells brick by brick (8 x 8 x 32 cells, cut off at the far
+// walls) instead of the whole grid's (i, j, k) order: a chunk of consecutive entries is then a
+// compact piece of the liquid, with about 0.6 neighbours outside it per cell where a chunk of whole
+// grid rows has 2.1, and still runs of up to 32 consecutive cells along z (resident solve at
+// 128^3: 2.70 -> 2.21 ms).  FP64 keeps the grid's order, whose chunks of the list its dot products
+// follow: they are the only thing that the order enters, in the last bit, and fp64 scalars carry
+// it into the pressure where the fp32 modes round it off.
+__device__ __forceinline__ int list_order(int mode, int n, int i, int j, int k) {
+    if (mode == kFp64) return (i * n + j) * n + k;
     const int i0 = i & ~7, j0 = j & ~7, k0 = k & ~31;
     const int bi = min(8, n - i0), bj = min(8, n - j0), bk = min(32, n - k0);
     return (i0 * n + j0 * bi) * n + k0 * bi * bj + ((i - i0) * bj + (j - j0)) * bk + (k - k0);
@@ -202,7 +206,7 @@ __global__ void k_prep_cells(PcgArgs A, uint32_t* pred) {
     const uint8_t flag = S.flags[c];
     int i, j, k;
     cell_ijk(D, c - D.c_begin, i, j, k);
-    pred[D.c_begin + list_order(n, i, j, k)] = flag == ARIEL_FLUID;
+    pred[D.c_begin + list_order(A.mode, n, i, j, k)] = flag == ARIEL_FLUID;
     if (flag != ARIEL_FLUID) {
         S.P[c] = 0.0f;
         if (S.P64) S.P64[c] = 0.0;
@@ -289,11 +293,18 @@ __device__ void pcg_tables(const PcgArgs& A, const uint32_t* scan) {
         ordered |= P.ordered;
     }
     const int any_ordered = __syncthreads_or(ordered);
-    const bool may = A.fast && G > 0 && !any_ordered && k <= kResMaxScenes;
-    auto max_cpb = [&](int s) { return res_max_cpb(A.mode, k, csz_s[s]); };
-    auto resident = [&](int s) {
-        return may && nch_s[s] <= kResMaxChunks && nch_s[s] <= max_cpb(s) * G;
-    };
+    // FP64 scenes are resident only alone: the grid order of their list gives blocks three times the
+    // halo, and several of them iterating together in the streaming kernel measured faster (six
+    // scenes of 32^3-96^3: 14.9 against 15.8 ms per step).
+    const bool may = A.fast && G > 0 && !any_ordered && k <= kResMaxScenes && (A.mode != kFp64 || k == 1);
+    auto max_cpb = [&](int s) { return res_max_cpb(A.mode, k, csz_s[s], nch_s[s]); };
+    auto fits = [&](int s) { return may && nch_s[s] <= kResBigChunks && nch_s[s] <= max_cpb(s) * G; };
+    // Where some scene has to stream, the others' cells cost little in its iterations, while a
+    // resident solve of their own comes on top: small scenes join it.
+    int stream = 0;
+    for (int s = threadIdx.x; s < k; s += kTableThreads) stream |= !fits(s);
+    const bool streams = __syncthreads_or(stream) != 0;
+    auto resident = [&](int s) { return fits(s) && !(streams && csz_s[s] == kChunkMin); };
     if (may) {
         for (int s = threadIdx.x; s < k; s += kTableThreads) {
             int rank = 0;
@@ -302,7 +313,7 @@ __device__ void pcg_tables(const PcgArgs& A, const uint32_t* scan) {
             if (resident(s))
                 for (int q = 0; q < 4; ++q) {
                     const int c = min(1 << q, max_cpb(s));
-                    atomicAdd(&need_s[res_class(k, csz_s[s])][q], (nch_s[s] + c - 1) / c);
+                    atomicAdd(&need_s[res_class(k, csz_s[s], nch_s[s])][q], (nch_s[s] + c - 1) / c);
                 }
         }
     }
@@ -315,7 +326,7 @@ __device__ void pcg_tables(const PcgArgs& A, const uint32_t* scan) {
         if (resident(s)) continue;
         acc += nch_s[s];
         ++nstream;
-        A.res[s] = make_int4(-1, 0, 0, 0);
+        A.res[s] = make_int4(kNotResident, 0, nch_s[s], 0);
     }
     chp[k] = acc;
     for (int cls = 0; cls < kResClasses; ++cls) {
@@ -323,13 +334,13 @@ __device__ void pcg_tables(const PcgArgs& A, const uint32_t* scan) {
         while (q < 3 && need_s[cls][q] > G) ++q;
         for (int i = 0; may && i < k; ++i) {
             const int s = order_s[i], nch = nch_s[s];
-            if (res_class(k, csz_s[s]) != cls || !resident(s)) continue;
+            if (res_class(k, csz_s[s], nch_s[s]) != cls || !resident(s)) continue;
             const int c = min(max(1 << q, (nch + G - 1) / G), max_cpb(s)), m = (nch + c - 1) / c;
             int g = 0;
             while (g < groups && fill_s[g] + m > G) ++g;
             if (g == groups) fill_s[groups++] = 0;
             A.res[s] = make_int4(g * G + fill_s[g], m, nch, partials);
-            A.res_count[32 * s] = 0u;
+            A.res_count[32 * s] = A.res_count[32 * s + 1] = 0u;
             fill_s[g] += m;
             partials += nch;
         }
@@ -360,7 +371,7 @@ __global__ void k_fl_write(PcgArgs A, const uint32_t* scan) {
     const SceneDev& D = S.scenes[find_scene(pref_s, S.k, c)];
     int i, j, k;
     cell_ijk(D, c - D.c_begin, i, j, k);
-    const uint32_t t = scan[D.c_begin + list_order(D.n, i, j, k)];
+    const uint32_t t = scan[D.c_begin + list_order(A.mode, D.n, i, j, k)];
     const_cast<uint32_t*>(A.fl)[t] = (uint32_t)c;
     uint4 r;
     r.x = (uint32_t)c;
@@ -1613,6 +1624,19 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_fast(PcgArgs A) {
         csz_s[i] = A.sc[i].csize;
     }
     __syncthreads();
+    if (MODE != kRef32) {
+        // the chunks of the scenes that are solved here: those that never were resident, and those
+        // whose halo did not fit
+        if (threadIdx.x == 0) {
+            long long acc = 0;
+            for (int i = 0; i < k; ++i) {
+                ch_s[i] = acc;
+                if (!L[i].resident) acc += (L[i].nf + csz_s[i] - 1) / csz_s[i];
+            }
+            ch_s[k] = acc;
+        }
+        __syncthreads();
+    }
     const long long nch = ch_s[k];
     const long long MC = A.max_chunks;
     // Two sets of partial sums used in turn: a block past one barrier may write its sums for the
@@ -2320,6 +2344,8 @@ static cudaError_t launch_res(const PcgArgs& A, cudaStream_t st) {
     if (e == cudaSuccess && (A.classes & 2)) e = coop_launch_res<MODE, 1>(A, st);
     if (e == cudaSuccess && (A.classes & 4)) e = coop_launch_res<MODE, 2>(A, st);
     if (e == cudaSuccess && (A.classes & 8)) e = coop_launch_res<MODE, 3>(A, st);
+    if constexpr (MODE == kMixed)
+        if (e == cudaSuccess && (A.classes & 16)) e = coop_launch_res<MODE, kResBig>(A, st);
     return e;
 }
 
@@ -2391,9 +2417,10 @@ int pcg_res_blocks(int device, int mode) {
     const void* const f64[] = {(const void*)k_pcg_res<kFp64, 0>, (const void*)k_pcg_res<kFp64, 1>,
                                (const void*)k_pcg_res<kFp64, 2>, (const void*)k_pcg_res<kFp64, 3>};
     const void* const f32[] = {(const void*)k_pcg_res<kMixed, 0>, (const void*)k_pcg_res<kMixed, 1>,
-                               (const void*)k_pcg_res<kMixed, 2>, (const void*)k_pcg_res<kMixed, 3>};
+                               (const void*)k_pcg_res<kMixed, 2>, (const void*)k_pcg_res<kMixed, 3>,
+                               (const void*)k_pcg_res<kMixed, kResBig>};
     bool ok = true;
-    for (int c = 0; c < kResClasses; ++c) ok = ok && fits(mode == kFp64 ? f64[c] : f32[c]);
+    for (int c = 0; c < (mode == kFp64 ? 4 : 5); ++c) ok = ok && fits(mode == kFp64 ? f64[c] : f32[c]);
     if (!ok) cudaGetLastError();
     return ok ? sms : 0;  // 0: no scene is resident
 }

@@ -42,8 +42,9 @@ struct PcgCtl {
     int all_done;
     int all_inner_done;
     int any_ordered;
-    int nvirt[4];  // block positions of the resident solve's classes (whole groups of gridDim.x)
+    int nvirt[5];  // block positions of the resident solve's classes (whole groups of gridDim.x)
     int nstream;   // scenes left to the streaming kernel
+    int pad[3];
 };
 
 struct Barrier {
@@ -71,13 +72,15 @@ struct PcgArgs {
     uint4* rec;                // per FLUID-list entry: (cell, neighbour mask, diagonal bits)
     const long long* fl_pref;  // k+1
     const long long* ch_pref;  // k+1 chunk begins (scenes of the resident solve have none)
+    uint32_t* hlist;           // resident solve, largest class: the blocks' halo positions
     const uint32_t* flscan;    // packed cell in list_order -> FLUID-list position
-    // resident solve: per scene (first block position, positions, chunks, first partial) or
-    // position -1 when it is not resident; one arrival counter per scene, 128 bytes apart
+    // resident solve: per scene (first block position, positions, chunks, first partial), or
+    // position kNotResident; one arrival counter per scene, 128 bytes apart, with a word that a
+    // block sets when its halo does not fit
     int4* res;
     unsigned* res_count;
     int res_blocks;            // its blocks (one per SM)
-    int all_resident;          // every scene fits the resident solve whatever its FLUID count
+    int all_resident;          // every scene fits the resident solve whatever its FLUID cells are
     int classes;               // bit c: some scene may be of class c
     // per-cell operator data (dense over packed cells)
     uint8_t* mask;   // bit d set: neighbour d (-x,+x,-y,+y,-z,+z) is FLUID
@@ -148,36 +151,49 @@ inline long long chunk_bound(long long cells) {
     return std::min(lo, std::max(kChunkTarget, hi));
 }
 // The resident solve: scenes of one chunk or more per block (one block per SM) whose cells fit its
-// shared memory together with slots for neighbours in other blocks, of which bricks of the
-// FLUID list's order have about 0.6 per cell.
-constexpr int kResMaxChunks = 320;
-constexpr int kResMaxScenes = 128;  // as the streaming fast kernel
+// shared memory together with slots for neighbours in other blocks.
+constexpr int kResMaxChunks = 320;   // what the reduction of a scene's partials reads in one go:
+constexpr int kResBigChunks = 608;   // up to two full-size chunks per block, and up to four
+constexpr int kResMaxScenes = 128;   // as the streaming fast kernel
 constexpr size_t kResSmem = 225 * 1024;  // all of an SM's but 2 KB for the static part
-// Slots for neighbours in other blocks beside a block's `cells` cells (positions fit 13 bits).
-__host__ __device__ constexpr int res_halo_slots(int mode, int cells) {
+// Slots for neighbours in other blocks beside a block's `cells` cells (positions fit 14 bits).
+__host__ __device__ constexpr int res_halo_slots(int mode, int cells, bool big) {
     const long long tb = mode == kFp64 ? 8 : 4;
-    const long long left = ((long long)kResSmem - 64 - cells * (5 * tb + 16)) / (tb + 4);
-    const long long most = 8190 - cells;
+    const long long left = ((long long)kResSmem - 64 - cells * ((big ? 3 : 5) * tb + 12)) / (tb + (big ? 0 : 4));
+    const long long most = 16380 - cells;
     return (int)(left < most ? left : most);
 }
 // Classes of resident scenes, one kernel each, by the rounds of one cell per thread that a chunk
 // takes and the chunks of a half block: a scene alone spreads over as many SMs as it can (one
 // chunk per half); with other scenes small chunks share a block, up to 4,096 cells, so that all
 // scenes iterate side by side (six 32^3-64^3 scenes: one group of blocks instead of four one
-// after another).
-constexpr int kResClasses = 4;
+// after another).  The last class takes scenes of more than two full-size chunks per SM, up to four
+// (MIXED): 0.6-1.2 M FLUID cells, whose (p, x) no longer fit beside the rest.
+constexpr int kNotResident = -(1 << 30);
+constexpr int kResClasses = 5;
+constexpr int kResBig = 4;
 __host__ __device__ constexpr int res_rounds(int c) { return c == 0 || c == 1 ? 2 : (c == 2 ? 4 : 8); }
-__host__ __device__ constexpr int res_chunks(int c) { return c == 1 ? 4 : (c == 2 ? 2 : 1); }
-__host__ __device__ constexpr int res_class(int scenes, int csize) {
-    return csize <= 512 ? (scenes == 1 ? 0 : 1) : (csize <= 1024 && scenes > 1 ? 2 : 3);
+__host__ __device__ constexpr int res_chunks(int c) { return c == 1 ? 4 : (c == 2 || c == kResBig ? 2 : 1); }
+__host__ __device__ constexpr int res_class(int scenes, int csize, int chunks) {
+    return chunks > kChunkTarget ? kResBig
+           : csize <= 512        ? (scenes == 1 ? 0 : 1)
+                                 : (csize <= 1024 && scenes > 1 ? 2 : 3);
 }
-__host__ __device__ constexpr bool res_fits(int mode, int cells) {
-    return 4 * res_halo_slots(mode, cells) >= 3 * cells;
+// Whether any cells of a chunk of this class find a slot for each neighbour (at most six).
+__host__ __device__ constexpr bool res_never_over(int mode, int csize, int cpb) {
+    return cpb > 0 && res_halo_slots(mode, cpb * csize, false) >= 6 * cpb * csize;
 }
-// Most chunks of `csize` cells that a block takes (0: none fits).
-__host__ __device__ constexpr int res_max_cpb(int mode, int scenes, int csize) {
-    int c = 2 * res_chunks(res_class(scenes, csize));
-    while (c > 0 && !res_fits(mode, c * csize)) c >>= 1;
+// Slots enough for the usual halo: about 0.6 neighbours in other blocks per cell, or in the grid
+// order of the FP64 list 2.1.
+__host__ __device__ constexpr bool res_fits(int mode, int cells, bool big) {
+    return 10 * res_halo_slots(mode, cells, big) >= (mode == kFp64 ? 21 : 8) * cells;
+}
+// Most chunks of `csize` cells that a block takes of a scene of `chunks` (0: none fits).
+__host__ __device__ constexpr int res_max_cpb(int mode, int scenes, int csize, int chunks) {
+    const int cls = res_class(scenes, csize, chunks);
+    if (cls == kResBig && mode != kMixed) return 0;
+    int c = 2 * res_chunks(cls);
+    while (c > 0 && !res_fits(mode, c * csize, cls == kResBig)) c >>= 1;
     return c;
 }
 constexpr int kBrickMaxCells = 2048;

@@ -1,24 +1,26 @@
-// pcg_resident.cuh -- the pressure solve of scenes of at most two chunks per SM (included by
-// pcg.cu after its helpers; FP64 and MIXED with the elementwise preconditioner).
+// pcg_resident.cuh -- the pressure solve of scenes whose chunks fit the SMs (included by pcg.cu after
+// its helpers; FP64 and MIXED with the elementwise preconditioner).
 //
 // k_pcg_fast keeps every scene of the launch in step: one grid barrier and one pass over all
 // partial sums per iteration, and every cell's state crosses L2 in every iteration.  A scene that
 // fits the SMs needs neither:
-//   - a block keeps its one or two chunks for the whole solve.  r, w, s stay in registers, p, x,
-//     u and the operator data in shared memory.  Only cells with a neighbour in another block
-//     write (r, w, s, pc) to L2, for those blocks to read.  Neighbours inside the block take the
-//     owner's u from shared memory, computed once per cell instead of once per neighbour;
+//   - a block keeps its chunks for the whole solve.  r, w, s stay in registers, p, x, u and the
+//     operator data in shared memory.  Only cells with a neighbour in another block write
+//     (r, w, s, pc) to L2, at their list position, for those blocks to read.  Neighbours inside
+//     the block take the owner's u from shared memory, computed once per cell instead of once per
+//     neighbour;
 //   - a block waits only for the blocks of its own scene, on the scene's own arrival counter.
 // Scenes are packed into groups of at most gridDim.x block positions; a block takes its position
 // of each group in turn, so small scenes run side by side and large ones one after another, each
 // out of shared memory, instead of all of them streaming through L2.
 //
-// MIXED to 1e-5, ms per solve, k_pcg_fast before -> here: 32^3 0.54 -> 0.33, 64^3 1.11 -> 0.68,
-// 128^3 3.90 -> 2.24 (10.0 -> 5.8 us per iteration); FP64 77^3 1.76 -> 1.30.  What an iteration of
-// the 128^3 dam break spends, in SM cycles of about 11,000: 2,400 own update and halo, 2,500 the
-// operator (shared-memory bandwidth: 11 words per cell), 900 block sums, 2,500-3,500 arrival and
-// wait (a release, a reduction and an acquire through L2), 2,200 reading 291 partials and the fp64
-// divisions of alpha and beta.  At 64^3 the last three are 5,500 of 6,700 cycles.
+// ms per solve, k_pcg_fast before -> here: MIXED 32^3 0.54 -> 0.30, 64^3 1.11 -> 0.66, 128^3 (0.50 M
+// FLUID cells) 3.90 -> 2.15 (10.0 -> 5.5 us per iteration), FP64 77^3 1.76 -> 1.48; eight scenes of
+// 32^3-128^3, two of them of 0.9 M cells, 24.5 -> 18.4.  What an iteration of the 128^3 dam break
+// spends, in SM cycles of about 10,800: 2,300 own update and halo, 2,400 the operator (shared
+// memory bandwidth: 11 words per cell), 900 block sums, 2,500-3,500 arrival and wait (a release, a
+// reduction and an acquire through L2), 2,200 reading 291 partials and the fp64 divisions of alpha
+// and beta.  At 64^3 the last three are 5,500 of 6,500 cycles.
 //
 // The arithmetic, the chunk of every cell, the entries of every thread and every summation tree
 // are those of k_pcg_fast, so both kernels give the same bits.
@@ -35,19 +37,18 @@ __device__ __forceinline__ double4 ldcg4(const double4* p) {
 // pollers make the barrier cheaper than two blocks per SM do (148 against 291 blocks: 2.2 against
 // 2.9 us for an arrival, the wait and the reading of three sums per chunk).
 constexpr int kResThreads = 2 * kPcgThreads;
-constexpr unsigned kResOut = 0x1fff;  // a neighbour without a slot of u
-static_assert(2 * kChunkMax + 2 * kChunkMax / 2 < (int)kResOut, "positions of u must fit 13 bits");
 
 // One block's part in one scene's solve: C chunks per half, Q rounds of one cell per thread in
-// each (csize <= 256 Q).  False when a wait gave up.
-template <int MODE, int Q, int C>
+// each (csize <= 256 Q).  BIG: blocks of up to four full-size chunks, whose (p, x), cell indices and
+// halo cells stay in global memory, read ahead of use.  False when a wait gave up.
+template <int MODE, int Q, int C, bool BIG>
 __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
     using T = typename VT<MODE>::T;
     using T2 = typename V2<T>::type;
     using T4 = typename V4<T>::type;
     constexpr int R = Q * C, kWarps = kPcgThreads / 32;
     // halo entries of a thread loaded ahead of alpha and beta, in registers
-    constexpr int kAhead = R <= 2 ? 2 : (MODE == kFp64 ? 2 : 5);
+    constexpr int kAhead = R <= 2 ? 2 : (MODE == kFp64 ? 2 : (BIG ? 4 : 5));
     const DevState& S = A.S;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int half = tid / kPcgThreads, htid = tid % kPcgThreads, hwid = htid >> 5;
@@ -80,18 +81,19 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
         o = (half + 2 * (q / Q)) * csize + i;
         return i < csize && o < blen;
     };
-    // Shared memory: per cell (p, x), the diagonal, pc, u, the cell index and three words of
-    // neighbour positions in u (x, y, z pairs of 13 bits; bit 26 of the first: some neighbour
-    // lies in another block); u continues with the halo -- the neighbours in other blocks --
-    // and a slot that stays 0 for neighbours that are not FLUID; the halo's cells.
-    const int cells = cpb * csize, hcap = res_halo_slots(MODE, cells), zero = cells + hcap;
-    T2* const px = reinterpret_cast<T2*>(dyn);
-    T* const dgs = reinterpret_cast<T*>(px + cells);
+    // Shared memory: per cell (p, x), the diagonal, pc, u and three words of neighbour positions in
+    // u (x, y, z pairs of 14 bits; bit 28 of the first: some neighbour lies in another block); u
+    // continues with the halo -- the neighbours in other blocks -- and a slot that stays 0 for
+    // neighbours that are not FLUID; the halo's list positions, where its owners publish.
+    const int cells = cpb * csize, hslots = res_halo_slots(MODE, cells, BIG);
+    const int hcap = BIG ? min(hslots, blen) : hslots, zero = cells + hcap;
+    T2* const px = BIG ? (T2*)A.vb + t0 : reinterpret_cast<T2*>(dyn);
+    T* const dgs = reinterpret_cast<T*>(dyn + (BIG ? 0 : sizeof(T2) * cells));
     T* const pcs = dgs + cells;
     T* const ub = pcs + cells;
-    uint32_t* const cs = reinterpret_cast<uint32_t*>(ub + zero + 1);
-    uint32_t* const nw = cs + cells;
-    uint32_t* const hcell = nw + 3 * cells;
+    uint32_t* const nw = reinterpret_cast<uint32_t*>(ub + zero + 1);
+    uint32_t* const hpos = BIG ? A.hlist + t0 : nw + 3 * cells;
+    const uint32_t* const cs = A.fl + t0;
     const unsigned arrivals = (unsigned)pl.y;
     unsigned* const count = A.res_count + 32 * (size_t)sc;
     unsigned epoch = 0;
@@ -172,8 +174,8 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
     // issues loads to overlap with it: after those of the partials, but before them where their
     // registers and those of the partials together would spill.
     auto sums = [&](int nsum, auto&& ahead, auto&& f) {
-        constexpr int kU = (kResMaxChunks + 31) / 32;
-        static_assert(kU <= 16, "scene_sum3 takes these partials in one go");
+        constexpr int kU = ((BIG ? kResBigChunks : kResMaxChunks) + 31) / 32;
+        // scene_sum3's order: partials a lane at a time, ascending
         if (R > 2) ahead();
         double x[kU];
         if (wid < nsum) {
@@ -216,7 +218,7 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
         bool out = false;
         auto code = [&](int d, int a, int b, int e) -> uint32_t {
             if (!((m >> d) & 1u)) return (uint32_t)zero;
-            const long long p = (long long)A.flscan[D.c_begin + list_order(n, a, b, e)] - t0;
+            const long long p = (long long)A.flscan[D.c_begin + list_order(MODE, n, a, b, e)] - t0;
             if (p >= 0 && p < blen) return (uint32_t)p;
             out = true;
             // one slot for each active lane, in lane order
@@ -225,24 +227,24 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
             int h = 0;
             if (lane == lead) h = atomicAdd(&s_nhalo, __popc(act));
             h = __shfl_sync(act, h, lead) + __popc(act & ((1u << lane) - 1u));
-            if (h >= hcap) return kResOut;
-            hcell[h] = c + (uint32_t)nb_off(d, n);
+            if (h < hcap) hpos[h] = (uint32_t)(p + t0);
             return (uint32_t)(cells + h);
         };
         const uint32_t x0 = code(0, i - 1, j, kk), x1 = code(1, i + 1, j, kk);
         const uint32_t y0 = code(2, i, j - 1, kk), y1 = code(3, i, j + 1, kk);
         const uint32_t z0 = code(4, i, j, kk - 1), z1 = code(5, i, j, kk + 1);
-        cs[o] = c;
         dgs[o] = dg;
         pcs[o] = pcv[c];
-        nw[o] = x0 | x1 << 13 | (out ? 1u << 26 : 0u);
-        nw[cells + o] = y0 | y1 << 13;
-        nw[2 * cells + o] = z0 | z1 << 13;
+        nw[o] = x0 | x1 << 14 | (out ? 1u << 28 : 0u);
+        nw[cells + o] = y0 | y1 << 14;
+        nw[2 * cells + o] = z0 | z1 << 14;
     }
-    // (every thread reads back only its own entries of cs, dgs, pcs, nw and px)
+    // (every thread reads back only its own entries of dgs, pcs, nw and px)
     __syncthreads();
-    const bool over = s_nhalo > hcap;  // some neighbours have no slot: read where needed
-    const int nhalo = min(s_nhalo, hcap);
+    const int nhalo = s_nhalo;
+    // More neighbours in other blocks than slots for them (liquid in sheets along the bricks' faces):
+    // the scene is left to the streaming kernel.  Its blocks learn of it at their first exchange.
+    if (tid == 0 && nhalo > hcap) atomicExch(count + 1, 1u);
 
     const T scale = (T)(1.0 / (double)D.ax_h);
     const int cap = A.max_iters > 0 ? A.max_iters : n * n * n;
@@ -274,6 +276,13 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
                 a1[j] += bv * bv;
             }
         if (!arrive_wait(2, a0, a1, a2)) return false;
+        if (outer == 0 && *(volatile unsigned*)(count + 1)) {
+            if (ch0 == 0 && tid == 0) {
+                A.res[sc].x = kNotResident;
+                atomicAdd(&A.ctl->nstream, 1);
+            }
+            return true;
+        }
         sums(2, [] {}, [&] {
             const double rr = total[0];
             if (outer == 0) st.bb = total[1];
@@ -328,7 +337,7 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
                     }
                 const T wv = acc * scale;
                 const T xv = MODE == kMixed ? (T)0 : (T)S.P64[c];
-                if (nw[o] >> 26) st4(Av0 + c, mk4<T>(rv, wv, (T)0, pcc));
+                if (nw[o] >> 28) st4(Av0 + t0 + o, mk4<T>(rv, wv, (T)0, pcc));
                 r[q] = rv;
                 w[q] = wv;
                 sv[q] = (T)0;
@@ -338,19 +347,40 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
             }
         }
         if (!arrive_wait(2, a0, a1, a2)) return false;
+        // BIG: this thread's halo positions, and (p, x) a group of rounds ahead of use
+        constexpr int kGroup = 4;
+        uint32_t hreg[BIG ? kAhead : 1];
+        T2 bn[BIG ? kGroup : 1];
+        auto load_px = [&](int q0) {
+            if constexpr (BIG) {
+#pragma unroll
+                for (int u = 0; u < kGroup; ++u) {
+                    int o;
+                    if (q0 + u < R && cell_of(q0 + u, o)) bn[u] = px[o];
+                }
+            }
+        };
+        if constexpr (BIG) {
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                const int h = tid + u * kResThreads;
+                hreg[u] = h < nhalo ? hpos[h] : 0u;
+            }
+        }
         // ---- iterations: k_pcg_fast's update of (r, w, s, p, x, u), one exchange each ---
         // The halo comes from L2 as its owners' (r, w, s, pc) of the last iteration; the loads
         // are issued as soon as the wait ends, ahead of alpha and beta.
         for (int it = 0;; ++it) {
             const T4* const Ac = (it & 1) ? Av1 : Av0;
-            T4* const An = (it & 1) ? Av0 : Av1;
+            T4* const mine = ((it & 1) ? Av0 : Av1) + t0;
             T4 eh[kAhead];
             auto load_halo = [&] {
 #pragma unroll
                 for (int u = 0; u < kAhead; ++u) {
                     const int h = tid + u * kResThreads;
-                    if (h < nhalo) eh[u] = ldcg4(Ac + hcell[h]);
+                    if (h < nhalo) eh[u] = ldcg4(Ac + (BIG ? hreg[u] : hpos[h]));
                 }
+                if (BIG) load_px(0);
             };
             if (it == 0)
                 sums(2, load_halo, [&] {
@@ -389,13 +419,21 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
                 if (h < nhalo) ub[cells + h] = u_of(eh[u]);
             }
             for (int h = tid + kAhead * kResThreads; h < nhalo; h += kResThreads)
-                ub[cells + h] = u_of(ldcg4(Ac + hcell[h]));
+                ub[cells + h] = u_of(ldcg4(Ac + hpos[h]));
+            T2 bc[BIG ? kGroup : 1];
 #pragma unroll
             for (int q = 0; q < R; ++q) {
+                if constexpr (BIG) {
+                    if (q % kGroup == 0) {
+#pragma unroll
+                        for (int u = 0; u < kGroup; ++u) bc[u] = bn[u];
+                        load_px(q + kGroup);
+                    }
+                }
                 int o;
                 if (cell_of(q, o)) {
                     const T pc = pcs[o];
-                    const T2 b = px[o];
+                    const T2 b = BIG ? bc[BIG ? q % kGroup : 0] : px[o];
                     const T s1 = w[q] + bt * sv[q];
                     const T ui = (r[q] * pc) * pc;
                     const T pv = ui + bt * b.x;
@@ -409,44 +447,35 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
             }
             __syncthreads();
             clear();
-            auto apply = [&](auto has_out) {
 #pragma unroll
-                for (int q = 0; q < R; ++q) {
-                    int o;
-                    if (cell_of(q, o)) {
-                        const uint32_t nb[3] = {nw[o], nw[cells + o], nw[2 * cells + o]};
-                        const T un = ub[o];
-                        T a = dgs[o] * un;
+            for (int q = 0; q < R; ++q) {
+                int o;
+                if (cell_of(q, o)) {
+                    const uint32_t nb[3] = {nw[o], nw[cells + o], nw[2 * cells + o]};
+                    const T un = ub[o];
+                    T a = dgs[o] * un;
 #pragma unroll
-                        for (int d = 0; d < 6; ++d) {
-                            const unsigned p = (d & 1 ? nb[d / 2] >> 13 : nb[d / 2]) & 0x1fffu;
-                            if (decltype(has_out)::value && p == kResOut)
-                                a -= u_of(ldcg4(Ac + cs[o] + nb_off(d, n)));
-                            else
-                                a -= ub[p];  // 0 where the neighbour is not FLUID
-                        }
-                        const T wn = a * scale;
-                        w[q] = wn;
-                        if (nb[0] >> 26) st4(An + cs[o], mk4<T>(r[q], wn, sv[q], pcs[o]));
-                        if (MODE == kMixed) {
-                            // products of two floats are exact in double, so the fused sums
-                            // round as the separate ones
-                            const double dr = (double)r[q], du = (double)un;
-                            a0[q / Q] = __fma_rn(dr, du, a0[q / Q]);
-                            a1[q / Q] = __fma_rn((double)wn, du, a1[q / Q]);
-                            a2[q / Q] = __fma_rn(dr, dr, a2[q / Q]);
-                        } else {
-                            a0[q / Q] += (double)r[q] * (double)un;
-                            a1[q / Q] += (double)wn * (double)un;
-                            a2[q / Q] += (double)r[q] * (double)r[q];
-                        }
+                    for (int d = 0; d < 3; ++d) {
+                        a -= ub[nb[d] & 0x3fffu];  // 0 where the neighbour is not FLUID
+                        a -= ub[nb[d] >> 14 & 0x3fffu];
+                    }
+                    const T wn = a * scale;
+                    w[q] = wn;
+                    if (nb[0] >> 28) st4(mine + o, mk4<T>(r[q], wn, sv[q], pcs[o]));
+                    if (MODE == kMixed) {
+                        // products of two floats are exact in double, so the fused sums round as
+                        // the separate ones
+                        const double dr = (double)r[q], du = (double)un;
+                        a0[q / Q] = __fma_rn(dr, du, a0[q / Q]);
+                        a1[q / Q] = __fma_rn((double)wn, du, a1[q / Q]);
+                        a2[q / Q] = __fma_rn(dr, dr, a2[q / Q]);
+                    } else {
+                        a0[q / Q] += (double)r[q] * (double)un;
+                        a1[q / Q] += (double)wn * (double)un;
+                        a2[q / Q] += (double)r[q] * (double)r[q];
                     }
                 }
-            };
-            if (over)
-                apply(std::true_type{});
-            else
-                apply(std::false_type{});
+            }
             if (!arrive_wait(3, a0, a1, a2)) return false;
         }
         __syncthreads();
@@ -505,7 +534,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_res(PcgArgs A) {
     if (blockIdx.x == 0)
         for (int s = tid; s < k; s += kResThreads) {
             const int4 e = A.res[s];
-            if (e.x < 0 || e.z > 0 || res_class(k, A.sc[s].csize) != CLASS) continue;
+            if (e.x < 0 || e.z > 0 || res_class(k, A.sc[s].csize, A.res[s].z) != CLASS) continue;
             // a scene without FLUID cells: solved as it is
             PcgScene o = load_sc(A.sc + s);
             o.outer = MODE == kMixed ? 1 : 0;
@@ -520,11 +549,11 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_res(PcgArgs A) {
         __syncthreads();
         for (int s = tid; s < k; s += kResThreads) {
             const int4 e = A.res[s];
-            if (v >= e.x && v < e.x + e.y && res_class(k, A.sc[s].csize) == CLASS) s_scene = s;
+            if (v >= e.x && v < e.x + e.y && res_class(k, A.sc[s].csize, A.res[s].z) == CLASS) s_scene = s;
         }
         __syncthreads();
         const int sc = s_scene;
         if (sc < 0) continue;  // no chunk for this block in this group
-        if (!res_scene<MODE, res_rounds(CLASS), res_chunks(CLASS)>(A, sc, v)) return;
+        if (!res_scene<MODE, res_rounds(CLASS), res_chunks(CLASS), CLASS == kResBig>(A, sc, v)) return;
     }
 }

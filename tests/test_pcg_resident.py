@@ -47,9 +47,10 @@ CASES = [
     (20, _first(20, 0)), (20, _first(20, 1)), (20, _first(20, 511)), (20, _first(20, 513)),
     (33, _first(33, 33 ** 3 - 700)), (60, _first(60, 148 * 512)), (60, _first(60, 148 * 512 + 1)),
     (61, _first(61, 296 * 512)), (61, _first(61, 296 * 512 + 1)),
-    # two full-size chunks per block, and one cell too many for them
+    # two full-size chunks per block, one cell more (up to four), four, and one cell too many
     (86, _first(86, 296 * 2048)), (86, _first(86, 296 * 2048 + 1)),
-    (134, _slabs(134)),
+    (107, _first(107, 592 * 2048)), (107, _first(107, 592 * 2048 + 1)),
+    (134, _slabs(134)), (160, _slabs(160)),
 ]
 
 
