@@ -568,8 +568,15 @@ __device__ __forceinline__ void p2g_row(const DevState& S, const SceneDev& D, in
                 if (z0 > z1) continue;
                 long long cb = D.c_begin + ((long long)sx * n + sy) * n;
                 uint32_t a = S.start[cb + z0], b = S.start[cb + z1 + 1];
+                // The next record is in flight while this one is weighed: the loop is a chain of
+                // dependent loads and tests otherwise (32^3 0.072 -> 0.053 ms, 64^3 0.161 -> 0.152,
+                // 77^3 0.294 -> 0.255, 128^3 0.907 -> 0.813, a 256^3 sphere 4.83 -> 4.53).  Its velocity is not loaded ahead:
+                // most records weigh nothing (16% slower at 128^3 when it was).
+                float4 qn = make_float4(0, 0, 0, 0);
+                if (a < b) qn = S.gpos4[a];
                 for (uint32_t t = a; t < b; ++t) {
-                    const float4 q = S.gpos4[t];
+                    const float4 q = qn;
+                    if (t + 1 < b) qn = S.gpos4[t + 1];
                     // sqrlength_xy2's sum, (dx^2 + dy^2) + dz^2, with the first term shared
                     const float2 d = __fadd2_rn(make_float2(q.x, q.y), nfxy);
                     const float2 s2 = __fmul2_rn(d, d);
@@ -615,12 +622,13 @@ __device__ __forceinline__ void p2g_row(const DevState& S, const SceneDev& D, in
 }
 
 // Thread -> group of F faces, with the group range cut in thirds that blocks take in turn;
-// `third` is the number of groups in one third (a multiple of the block size).  Five blocks per
-// SM (48 registers; 50 unbounded, which the allocator rounds to four blocks): the latency-bound
-// gather gains from the extra warps (64^3 16%, 160^3 4%, 256^3 5% faster; 128^3 level to 3%
-// faster; six blocks, at 40 registers with spills, are slower).
+// `third` is the number of groups in one third (a multiple of the block size).  Four blocks of 256
+// per SM: the record loaded ahead in p2g_row needs 49 to 64 registers.  Five blocks spill it (4% to
+// 8% slower at 32^3, 77^3 and 128^3, 3% at 256^3; 4% faster only at 64^3, where it saves a wave);
+// three are level up to 128^3 and 6% slower at 256^3; blocks of 128 find less of each other's
+// records in L1 (1% to 15% slower).
 template <int F>
-__global__ void __launch_bounds__(kBlock, 5) k_p2g(DevState S, long long third) {
+__global__ void __launch_bounds__(kBlock, 4) k_p2g(DevState S, long long third) {
     kernel_begin();
     SCENE_PREFIX(S.f_pref);
     const long long grp = (long long)(blockIdx.x % 3) * third + (long long)(blockIdx.x / 3) * blockDim.x + threadIdx.x;
