@@ -901,7 +901,6 @@ ariel_status new_sim(const AsimSceneDesc* descs, int k, const AsimParams& prm, c
         for (auto& e : set) cudaEventCreate(&e);
     cudaEventCreate(&s->tb);
     cudaEventCreate(&s->te);
-    host_pool_retain();
     *out = s;
     return ARIEL_OK;
 }
@@ -917,7 +916,6 @@ void delete_sim(ariel_sim* s) {
     cudaEventDestroy(s->te);
     if (s->own_stream) cudaStreamDestroy(s->stream);
     delete s;
-    host_pool_release();
 }
 
 }  // namespace hostimpl
@@ -1427,9 +1425,9 @@ ariel_status ariel_set_grid(ariel_sim* s, int32_t scene, int32_t which, const vo
             if (in[i] < 0 || in[i] > 2) return ARIEL_ERR_INVALID_ARG;
             f[i] = (uint8_t)in[i];
         }
-        ARIEL_CUDA(upload(s->stream, d, f.data(), elems));
+        ARIEL_CUDA(copy_sync(s->stream, d, f.data(), elems, cudaMemcpyHostToDevice));
     } else {
-        ARIEL_CUDA(upload(s->stream, d, buf, elems * esize));
+        ARIEL_CUDA(copy_sync(s->stream, d, buf, elems * esize, cudaMemcpyHostToDevice));
     }
     return ARIEL_OK;
 }

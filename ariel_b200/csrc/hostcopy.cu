@@ -1,13 +1,19 @@
-// hostcopy.cu -- copies between device memory and ordinary (pageable) host buffers.
+// hostcopy.cu -- copies from device memory to ordinary (pageable) host buffers.
 //
-// A plain cudaMemcpyAsync to pageable memory is staged by one thread inside the driver, which
-// also takes the page faults of a fresh result array: 211,584 particles came out at 3 GB/s.
-// Here the copy goes through pinned chunks: the device fills them at the link's rate while up to
-// kWorkers host threads move the finished ones, so that the host's share (the memory copy and
-// the first touch of the pages) runs in parallel and beside the transfer.
+// The driver's staging writes a buffer whose pages are there at 17 GB/s (10 MB), but a fresh one,
+// such as a newly allocated result array, at 2.3 GB/s: its one thread takes a page fault every
+// 4 KB.  Here several threads take those faults first, and the driver copies what is ready behind
+// them: 10 MB into fresh pages 4.55 -> 2.3 ms, 2.5 MB 1.16 -> 0.8 ms, 40 MB 18.2 -> 6.4 ms.
+// Nothing is allocated: pinned chunks of the framework's own reach the same rates, but pinning
+// 8 MB of them cost the first copy after a handle's creation 4 to 8 ms.
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
 #include <atomic>
-#include <mutex>
+#include <cstdint>
+#include <memory>
+#include <new>
 #include <system_error>
 #include <thread>
 #include <vector>
@@ -18,93 +24,34 @@ namespace ariel {
 namespace hostimpl {
 namespace {
 
-constexpr size_t kChunk = 512 * 1024;
-constexpr size_t kDirect = 192 * 1024;  // below this the driver's own staging is as fast
-constexpr int kSlots = 16;              // chunks of one copy in flight
-constexpr int kPool = 4 * kSlots;       // pinned chunks kept for the next copies: 32 MB at most
-constexpr int kWorkers = 4;             // host threads of one copy, the caller among them
+constexpr size_t kPart = 512 * 1024;  // what a thread makes ready at a time
+// Fresh bytes below which the faults are left to the driver's thread (1 MB is level, 0.48 ms;
+// 512 KB is 0.25 ms either way).
+constexpr size_t kFresh = 1024 * 1024;
+// Ready bytes that the caller copies at a time while others still work (the copies wait for
+// the device one by one: 512 KB each reach 10.5 GB/s, 2.5 MB 15.8).
+constexpr size_t kRun = 2 * 1024 * 1024;
+constexpr int kWorkers = 4;  // host threads of one copy, the caller among them
 
-struct Slot {
-    void* p = nullptr;
-    cudaEvent_t ev = nullptr;
-    int device = 0;
-};
-
-// Pinned chunks shared by all handles.  A copy takes what it needs and gives it back; chunks
-// beyond kPool are freed at once, the others with the last handle.
-struct Pool {
-    std::mutex m;
-    std::vector<Slot> free;
-    int handles = 0;
-};
-Pool& pool() {
-    static Pool* p = new Pool;  // never destroyed: threads may outlive static destruction
-    return *p;
-}
-
-void drop(const Slot& s) {
-    cudaEventDestroy(s.ev);
-    cudaFreeHost(s.p);
-}
-
-struct Lease {
-    std::vector<Slot> slots;
-    // Up to `n` chunks for the current device; fewer (or none) when pinned memory is short.
-    Lease(int device, int n) {
-        Pool& P = pool();
-        {
-            std::lock_guard<std::mutex> l(P.m);
-            for (size_t i = P.free.size(); i-- > 0 && (int)slots.size() < n;)
-                if (P.free[i].device == device) {
-                    slots.push_back(P.free[i]);
-                    P.free.erase(P.free.begin() + (long)i);
-                }
-        }
-        while ((int)slots.size() < n) {
-            Slot s;
-            s.device = device;
-            if (cudaHostAlloc(&s.p, kChunk, cudaHostAllocDefault) != cudaSuccess) {
-                cudaGetLastError();
-                break;
-            }
-            if (cudaEventCreateWithFlags(&s.ev, cudaEventDisableTiming) != cudaSuccess) {
-                cudaGetLastError();
-                cudaFreeHost(s.p);
-                break;
-            }
-            slots.push_back(s);
-        }
-    }
-    ~Lease() {
-        Pool& P = pool();
-        std::lock_guard<std::mutex> l(P.m);
-        for (const Slot& s : slots) {
-            if (P.handles > 0 && (int)P.free.size() < kPool)
-                P.free.push_back(s);
-            else
-                drop(s);
-        }
-    }
-};
-
-// Runs `work` on the caller and `extra` more threads (fewer if they cannot be started).
-template <class F>
-void on_threads(int device, int extra, F&& work) {
+// Joins its threads when it goes.
+struct Helpers {
     std::vector<std::thread> t;
-    t.reserve((size_t)extra);
-    for (int i = 0; i < extra; ++i) {
-        try {
-            t.emplace_back([&work, device] {
-                cudaSetDevice(device);
-                work();
-            });
-        } catch (const std::system_error&) {
-            break;
+    // up to `n` threads (fewer if they cannot be started) that run `work`
+    template <class F>
+    Helpers(int n, const F& work) {
+        t.reserve((size_t)std::max(n, 0));
+        for (int i = 0; i < n; ++i) {
+            try {
+                t.emplace_back(work);
+            } catch (const std::system_error&) {
+                break;
+            }
         }
     }
-    work();
-    for (auto& x : t) x.join();
-}
+    ~Helpers() {
+        for (auto& x : t) x.join();
+    }
+};
 
 bool pinned_host(const void* p) {
     cudaPointerAttributes a{};
@@ -115,129 +62,111 @@ bool pinned_host(const void* p) {
     return a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeManaged;
 }
 
+// Whether most pages of [p, p + bytes) (at most kPart of it is looked at) are not mapped yet.
+bool fresh_pages(const char* p, size_t bytes, size_t page) {
+    unsigned char v[kPart / 4096 + 2];
+    const uintptr_t a = (uintptr_t)p & ~(uintptr_t)(page - 1);
+    const uintptr_t b = (uintptr_t)p + std::min(bytes, kPart);
+    const size_t n = (b - a + page - 1) / page;
+    if (page < 4096 || n > sizeof(v) || mincore((void*)a, b - a, v) != 0) return false;
+    size_t out = 0;
+    for (size_t i = 0; i < n; ++i) out += (v[i] & 1) == 0;
+    return 2 * out > n;
+}
+
+bool fresh(const char* p, size_t bytes, size_t page) {
+    const size_t tail = bytes > kPart ? bytes - kPart : 0;
+    return !pinned_host(p) && (fresh_pages(p, bytes, page) || fresh_pages(p + tail, bytes - tail, page));
+}
+
+// A write fault on every page of [p, p + bytes); the bytes keep their values.
+void touch(char* p, size_t bytes, size_t page) {
+    for (size_t o = 0; o < bytes; o += page) __atomic_fetch_or(p + o, (char)0, __ATOMIC_RELAXED);
+    __atomic_fetch_or(p + bytes - 1, (char)0, __ATOMIC_RELAXED);
+}
+
+// Device bytes to host int32 through a buffer of the bytes.
+cudaError_t download_i32(cudaStream_t st, const HostPiece& h) {
+    const std::unique_ptr<uint8_t[]> f(new (std::nothrow) uint8_t[h.bytes]);
+    if (!f) return cudaErrorMemoryAllocation;
+    cudaError_t e = download(st, {{f.get(), h.dev, h.bytes}});
+    if (e != cudaSuccess) return e;
+    int32_t* const out = static_cast<int32_t*>(h.host);
+    constexpr size_t kElems = kPart / sizeof(int32_t);
+    const size_t n = (h.bytes + kElems - 1) / kElems;
+    std::atomic<size_t> next{0};
+    auto work = [&] {
+        for (size_t i = next++; i < n; i = next++)
+            for (size_t j = i * kElems, end = std::min(j + kElems, h.bytes); j < end; ++j) out[j] = f[j];
+    };
+    Helpers helpers((int)std::min<size_t>(kWorkers, n) - 1, work);
+    work();
+    return cudaSuccess;
+}
+
 }  // namespace
-
-void host_pool_retain() {
-    std::lock_guard<std::mutex> l(pool().m);
-    ++pool().handles;
-}
-
-void host_pool_release() {
-    Pool& P = pool();
-    std::lock_guard<std::mutex> l(P.m);
-    if (--P.handles > 0) return;
-    for (const Slot& s : P.free) drop(s);
-    P.free.clear();
-}
 
 cudaError_t download(cudaStream_t st, const std::vector<HostPiece>& pieces) {
     struct Part {
         const HostPiece* h;
         size_t off, bytes;
     };
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
     std::vector<Part> parts;
-    cudaError_t e = cudaSuccess;
     size_t total = 0;
-    for (const HostPiece& h : pieces) total += h.bytes;
+    for (const HostPiece& h : pieces)
+        if (!h.to_i32) total += h.bytes;
+    std::vector<const HostPiece*> plain;
     for (const HostPiece& h : pieces) {
-        if (h.bytes == 0) continue;
-        if (!h.to_i32 && (total < kDirect || pinned_host(h.host))) {
-            e = cudaMemcpyAsync(h.host, h.dev, h.bytes, cudaMemcpyDeviceToHost, st);
-            if (e != cudaSuccess) return e;
-            continue;
-        }
-        for (size_t o = 0; o < h.bytes; o += kChunk) parts.push_back({&h, o, std::min(kChunk, h.bytes - o)});
+        if (h.bytes == 0 || h.to_i32) continue;
+        if (total >= kFresh && fresh(static_cast<const char*>(h.host), h.bytes, page))
+            for (size_t o = 0; o < h.bytes; o += kPart) parts.push_back({&h, o, std::min(kPart, h.bytes - o)});
+        else
+            plain.push_back(&h);
     }
-    if (parts.empty()) return cudaStreamSynchronize(st);
-    int device = 0;
-    cudaGetDevice(&device);
-    const int n = (int)parts.size();
-    Lease lease(device, std::min(n, kSlots));
-    const int m = (int)lease.slots.size();
-    if (m == 0) {
-        // no pinned memory to be had: the driver's staging
-        for (const HostPiece& h : pieces) {
-            if (h.to_i32) {
-                std::vector<uint8_t> f(h.bytes);
-                e = copy_sync(st, f.data(), h.dev, h.bytes, cudaMemcpyDeviceToHost);
-                if (e != cudaSuccess) return e;
-                for (size_t i = 0; i < h.bytes; ++i) static_cast<int32_t*>(h.host)[i] = f[i];
-            } else {
-                e = copy_sync(st, h.host, h.dev, h.bytes, cudaMemcpyDeviceToHost);
-                if (e != cudaSuccess) return e;
+    const size_t n = parts.size();
+    std::vector<std::atomic<bool>> ready(n);
+    std::atomic<size_t> next{0};
+    cudaError_t e = cudaSuccess;
+    {
+        auto take = [&] {
+            const size_t i = next++;
+            if (i >= n) return false;
+            touch(static_cast<char*>(parts[i].h->host) + parts[i].off, parts[i].bytes, page);
+            ready[i].store(true, std::memory_order_release);
+            return true;
+        };
+        Helpers helpers((int)std::min<size_t>(kWorkers, (n + 1) / 2) - 1, [&] {
+            while (take()) {
             }
-        }
-        return cudaStreamSynchronize(st);
-    }
-    std::atomic<int> err{0}, next{0};
-    std::vector<std::atomic<int>> issued((size_t)m);  // the part whose copy into the slot is queued
-    auto issue = [&](int i) {
-        const Slot& s = lease.slots[(size_t)(i % m)];
-        const Part& p = parts[(size_t)i];
-        cudaError_t r = cudaMemcpyAsync(s.p, static_cast<const char*>(p.h->dev) + p.off, p.bytes, cudaMemcpyDeviceToHost, st);
-        if (r == cudaSuccess) r = cudaEventRecord(s.ev, st);
-        if (r != cudaSuccess) err = (int)r;
-        issued[(size_t)(i % m)].store(i, std::memory_order_release);
-    };
-    for (auto& x : issued) x = -1;
-    for (int i = 0; i < m; ++i) issue(i);
-    on_threads(device, std::min(kWorkers, (n + 1) / 2) - 1, [&] {
-        for (int i = next++; i < n; i = next++) {
-            // (the part before it in its slot was taken earlier, so its issuer is at work)
-            while (issued[(size_t)(i % m)].load(std::memory_order_acquire) != i) std::this_thread::yield();
-            const Slot& s = lease.slots[(size_t)(i % m)];
-            const Part& p = parts[(size_t)i];
-            if (err == 0) {
-                const cudaError_t r = cudaEventSynchronize(s.ev);
-                if (r != cudaSuccess) err = (int)r;
-            }
-            if (err == 0) {
-                if (p.h->to_i32) {
-                    const uint8_t* f = static_cast<const uint8_t*>(s.p);
-                    int32_t* o = static_cast<int32_t*>(p.h->host) + p.off;
-                    for (size_t j = 0; j < p.bytes; ++j) o[j] = f[j];
-                } else {
-                    std::memcpy(static_cast<char*>(p.h->host) + p.off, s.p, p.bytes);
+        });
+        size_t done = 0;  // parts copied so far
+        // copies the parts from `done` on that are ready, a piece at a time
+        auto flush = [&](bool all) {
+            while (done < n && e == cudaSuccess) {
+                const HostPiece* h = parts[done].h;
+                size_t r = done, bytes = 0;
+                for (; r < n && parts[r].h == h; ++r) {
+                    while (all && !ready[r].load(std::memory_order_acquire)) std::this_thread::yield();
+                    if (!ready[r].load(std::memory_order_acquire)) break;
+                    bytes += parts[r].bytes;
                 }
+                if (bytes == 0 || (!all && bytes < kRun)) return;
+                const size_t o = parts[done].off;
+                e = cudaMemcpyAsync(static_cast<char*>(h->host) + o, static_cast<const char*>(h->dev) + o, bytes,
+                                    cudaMemcpyDeviceToHost, st);
+                done = r;
             }
-            if (i + m < n) issue(i + m);
-        }
-    });
-    e = cudaStreamSynchronize(st);
-    return err ? (cudaError_t)err.load() : e;
-}
-
-cudaError_t upload(cudaStream_t st, void* dev, const void* host, size_t bytes) {
-    if (bytes < kDirect || pinned_host(host)) return copy_sync(st, dev, host, bytes, cudaMemcpyHostToDevice);
-    int device = 0;
-    cudaGetDevice(&device);
-    const int n = (int)((bytes + kChunk - 1) / kChunk);
-    Lease lease(device, std::min(n, kSlots));
-    const int m = (int)lease.slots.size();
-    if (m == 0) return copy_sync(st, dev, host, bytes, cudaMemcpyHostToDevice);
-    std::atomic<int> err{0}, next{0};
-    std::vector<std::atomic<int>> queued((size_t)m);  // the last part queued from the slot
-    for (auto& x : queued) x = -1;
-    on_threads(device, std::min(kWorkers, (n + 1) / 2) - 1, [&] {
-        for (int i = next++; i < n; i = next++) {
-            const Slot& s = lease.slots[(size_t)(i % m)];
-            const size_t off = (size_t)i * kChunk, len = std::min(kChunk, bytes - off);
-            cudaError_t r = cudaSuccess;
-            if (i >= m) {
-                while (queued[(size_t)(i % m)].load(std::memory_order_acquire) != i - m) std::this_thread::yield();
-                r = cudaEventSynchronize(s.ev);
-            }
-            if (r == cudaSuccess && err == 0) {
-                std::memcpy(s.p, static_cast<const char*>(host) + off, len);
-                r = cudaMemcpyAsync(static_cast<char*>(dev) + off, s.p, len, cudaMemcpyHostToDevice, st);
-                if (r == cudaSuccess) r = cudaEventRecord(s.ev, st);
-            }
-            if (r != cudaSuccess) err = (int)r;
-            queued[(size_t)(i % m)].store(i, std::memory_order_release);
-        }
-    });
-    const cudaError_t e = cudaStreamSynchronize(st);
-    return err ? (cudaError_t)err.load() : e;
+        };
+        while (take()) flush(false);
+        flush(true);
+        for (const HostPiece* h : plain)
+            if (e == cudaSuccess) e = cudaMemcpyAsync(h->host, h->dev, h->bytes, cudaMemcpyDeviceToHost, st);
+    }
+    for (const HostPiece& h : pieces)
+        if (h.to_i32 && h.bytes && e == cudaSuccess) e = download_i32(st, h);
+    const cudaError_t se = cudaStreamSynchronize(st);
+    return e != cudaSuccess ? e : se;
 }
 
 }  // namespace hostimpl

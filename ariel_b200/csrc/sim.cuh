@@ -133,8 +133,8 @@ namespace hostimpl {
 ariel_status map_cuda_error(cudaError_t e, const char* what = "");
 cudaError_t copy_sync(cudaStream_t st, void* dst, const void* src, size_t bytes, cudaMemcpyKind kind);
 
-// Copies between device memory and ordinary host buffers through pinned chunks (hostcopy.cu);
-// both wait for the stream.  `to_i32`: device bytes become host int32 (cell types).
+// Copies from device memory to host buffers of any kind (hostcopy.cu); waits for the stream.
+// `to_i32`: device bytes become host int32 (cell types).
 struct HostPiece {
     void* host;
     const void* dev;
@@ -142,10 +142,6 @@ struct HostPiece {
     bool to_i32 = false;
 };
 cudaError_t download(cudaStream_t st, const std::vector<HostPiece>& pieces);
-cudaError_t upload(cudaStream_t st, void* dev, const void* host, size_t bytes);
-// The pinned chunks are kept while there are handles.
-void host_pool_retain();
-void host_pool_release();
 
 ariel_status validate(const AsimSceneDesc& d);
 SceneDev make_scene(const AsimSceneDesc& d, const AsimParams& p);

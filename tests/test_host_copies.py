@@ -1,7 +1,7 @@
 """Copies between device state and ordinary host buffers (csrc/hostcopy.cu): what is set is what
-is read back, around the sizes where the copy changes its form (the driver's staging below 192 KB,
-then pinned chunks of 512 KB, sixteen of them in flight), from several threads at once, and with
-the particles equal to those of the pinned-buffer path."""
+is read back, around the sizes where the copy changes its form (the driver's staging alone below
+1 MB or into mapped pages, then behind threads that map the pages in parts of 512 KB), from several
+threads at once, and with the particles equal to those of the pinned-buffer path."""
 import threading
 
 import numpy as np
