@@ -803,8 +803,13 @@ __device__ __forceinline__ void column_slots(const DevState& S, const SceneDev& 
 // so usually 2 per axis), testing only distance, records the few candidates in ascending slot
 // order -- the reference's summation order -- and then evaluates them with the reference's
 // exact arithmetic.  Neighbours outside the radius contribute exactly nothing.
-// Five blocks per SM (51 registers, a 12-byte spill): 1-2% faster than four.
-__global__ void __launch_bounds__(kBlock, 5) k_resample_spring(DevState S) {
+// While a candidate is evaluated the next one's record is loaded, which each candidate waited
+// for before (both kernels together, with four blocks per SM for the first:
+// 32^3 0.149 -> 0.141 ms, 64^3 0.317 -> 0.299, 77^3 0.501 -> 0.487, 128^3 1.687 -> 1.681, a 256^3
+// sphere 3.15 -> 3.17).  Five blocks (51 registers) spill the record: 3% slower at 32^3 and 64^3,
+// 1% faster from 128^3 on.  Groups of four test loads with a clamped index, in place of an unrolled
+// loop's remainder, are 4% slower.
+__global__ void __launch_bounds__(kBlock, 4) k_resample_spring(DevState S) {
     kernel_begin();
     SCENE_PREFIX(S.p_pref);
     __shared__ uint32_t lst[kResList][kBlock];
@@ -828,10 +833,9 @@ __global__ void __launch_bounds__(kBlock, 5) k_resample_spring(DevState S) {
     uint32_t draws = 0;
     float3 spring = make_float3(0, 0, 0);
     // particleresampler.inl:58-78 for one neighbour slot t (the particle itself is skipped)
-    auto eval = [&](uint32_t t) {
+    auto eval = [&](uint32_t t, float4 q) {
         if (t == (uint32_t)s) return;
         const float springforce = 50.0f;
-        float4 q = S.spos4[t];
         float3 d = make_float3(p4.x - q.x, p4.y - q.y, p4.z - q.z);
         float dist = sqrtf(gdot3(d, d));
         float w = springforce * q.w * smooth_fast(dist * dist, re, D.re_pow2, D.re_inv_hh);
@@ -852,6 +856,21 @@ __global__ void __launch_bounds__(kBlock, 5) k_resample_spring(DevState S) {
             spring.z += 0.05f * re / dt * 0.0f;
         }
     };
+    int nl = 0;
+    auto run_list = [&] {
+        if (nl == 0) return;
+        uint32_t t = lst[0][me];
+        float4 q = S.spos4[t];
+        for (int i = 0; i < nl; ++i) {
+            const uint32_t tc = t;
+            const float4 qc = q;
+            if (i + 1 < nl) {
+                t = lst[i + 1][me];
+                q = S.spos4[t];
+            }
+            eval(tc, qc);
+        }
+    };
     int xl, xh, yl, yh, zl, zh;
     // of the reference's 27 cells, only those within the candidate radius (5% margin over the
     // test below, for the rounding of the cell boxes)
@@ -866,7 +885,6 @@ __global__ void __launch_bounds__(kBlock, 5) k_resample_spring(DevState S) {
         axis_cells(p4.y, min((int)gy, n - 1), n, ch, lim, yl, yh);
         axis_cells(p4.z, min((int)gz, n - 1), n, ch, lim, zl, zh);
     }
-    int nl = 0;
     const float2 npxy = make_float2(-p4.x, -p4.y);
     if (zl <= zh) {
         for (int sx = xl; sx <= xh; ++sx)
@@ -885,13 +903,13 @@ __global__ void __launch_bounds__(kBlock, 5) k_resample_spring(DevState S) {
                         nl += sqrlength_xy2(q, npxy, p4.z) < near2 ? 1 : 0;
                     }
                     if (nl == kResList) {
-                        for (int i = 0; i < nl; ++i) eval(lst[i][me]);
+                        run_list();
                         nl = 0;
                     }
                 }
             }
     }
-    for (int i = 0; i < nl; ++i) eval(lst[i][me]);
+    run_list();
     float4 t4;
     t4.x = p4.x + dt * spring.x;
     t4.y = p4.y + dt * spring.y;
@@ -920,16 +938,29 @@ __global__ void __launch_bounds__(kBlock, 4) k_resample_velocity(DevState S) {
     float wsum = 0.0f;
     float3 ru = make_float3(0, 0, 0);
     // Resample (particleresampler.inl:133-141) for one neighbour slot
-    auto eval = [&](uint32_t q) {
-        float4 nv = S.svel4[q];
+    auto eval = [&](float4 nv, float4 np) {
         if (type_of(nv) != ARIEL_FLUID) return;
-        float4 np = S.spos4[q];
         float dist2 = sqrlength(t.x, t.y, t.z, np.x, np.y, np.z);
         float w = np.w * sharpen_k(dist2, re);
         ru.x = ru.x + w * nv.x;
         ru.y = ru.y + w * nv.y;
         ru.z = ru.z + w * nv.z;
         wsum += w;
+    };
+    int nl = 0;
+    auto run_list = [&] {
+        if (nl == 0) return;
+        uint32_t q = lst[0][me];
+        float4 v = S.svel4[q], p = S.spos4[q];
+        for (int i = 0; i < nl; ++i) {
+            const float4 vc = v, pc = p;
+            if (i + 1 < nl) {
+                q = lst[i + 1][me];
+                v = S.svel4[q];
+                p = S.spos4[q];
+            }
+            eval(vc, pc);
+        }
     };
     int xl, xh, yl, yh, zl, zh;
     const float ch = 1.0f / maxd, lim = 1.05f * re2;
@@ -943,7 +974,6 @@ __global__ void __launch_bounds__(kBlock, 4) k_resample_velocity(DevState S) {
         axis_cells(t.y, min((int)gy, n - 1), n, ch, lim, yl, yh);
         axis_cells(t.z, min((int)gz, n - 1), n, ch, lim, zl, zh);
     }
-    int nl = 0;
     const float2 ntxy = make_float2(-t.x, -t.y);
     if (zl <= zh) {
         for (int sx = xl; sx <= xh; ++sx)
@@ -962,13 +992,13 @@ __global__ void __launch_bounds__(kBlock, 4) k_resample_velocity(DevState S) {
                         nl += sqrlength_xy2(np, ntxy, t.z) < re2 ? 1 : 0;
                     }
                     if (nl == kResList) {
-                        for (int i = 0; i < nl; ++i) eval(lst[i][me]);
+                        run_list();
                         nl = 0;
                     }
                 }
             }
     }
-    for (int i = 0; i < nl; ++i) eval(lst[i][me]);
+    run_list();
     if (wsum != 0.0f)
         ru = f3div(ru, wsum);
     else
