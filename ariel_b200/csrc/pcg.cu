@@ -1639,6 +1639,19 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_fast(PcgArgs A) {
     }
     const long long nch = ch_s[k];
     const long long MC = A.max_chunks;
+    // The chunk that this block takes j-th in a pass, nch past the last.  With `rev` the streamed
+    // chunks come in descending order: successive iterations of the single-reduction path go
+    // through them in alternate directions, so that an iteration begins with what the last one
+    // left in L2.  A state larger than L2 (56 B per cell; 158 MB for a 256^3 sphere's 2.8 M cells)
+    // is evicted just before its use when every pass starts at the same end: 17.9 -> 16.6 ms a
+    // solve.  The sums are kept by chunk, so their order does not change.
+    const int own_chunks = nch > blockIdx.x ? (int)((nch - 1 - blockIdx.x) / gridDim.x) + 1 : 0;
+    bool rev = false;
+    auto chunk_no = [&](int j) -> long long {
+        if (j >= own_chunks) return nch;
+        if (rev && j >= kFlCacheChunks) j = own_chunks - 1 - (j - kFlCacheChunks);
+        return blockIdx.x + (long long)j * gridDim.x;
+    };
     // Two sets of partial sums used in turn: a block past one barrier may write its sums for the
     // next while a slower block still reads those of the last.
     auto part = [&](unsigned e, int i) { return A.partial + ((e & 1u) * 3 + i) * MC; };
@@ -1664,7 +1677,7 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_fast(PcgArgs A) {
             v1 = warp_sum(v1);
             v2 = warp_sum(v2);
             if (lane == 0) {
-                const long long ch = blockIdx.x + (long long)(jpend0 + jj) * gridDim.x;
+                const long long ch = chunk_no(jpend0 + jj);
                 part(epoch, 0)[ch] = v0;
                 part(epoch, 1)[ch] = v1;
                 part(epoch, 2)[ch] = v2;
@@ -1674,7 +1687,7 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_fast(PcgArgs A) {
         npend = 0;
     };
     auto chunk_of = [&](int j, int& s, long long& t0, long long& t1) -> bool {
-        long long ch = blockIdx.x + (long long)j * gridDim.x;
+        const long long ch = chunk_no(j);
         if (ch >= nch) {
             flush();  // every chunk pass ends here
             return false;
@@ -1891,6 +1904,7 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_fast(PcgArgs A) {
                 return true;
             });
             for (int it = 0;; ++it) {
+                rev = !rev;
                 const T4* Ac = (it & 1) ? Av1 : Av0;
                 T4* An = (it & 1) ? Av0 : Av1;
                 const int step = kIlp * (int)blockDim.x;
@@ -1910,7 +1924,7 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_fast(PcgArgs A) {
                         return true;
                     }
                     for (int jj = p.j + 1;; ++jj) {
-                        const long long ch = blockIdx.x + (long long)jj * gridDim.x;
+                        const long long ch = chunk_no(jj);
                         if (ch >= nch) return false;
                         const int s2 = find_scene(ch_s, k, ch);
                         const long long cs = csz_s[s2];
