@@ -1,11 +1,14 @@
 // pcg.cu -- the pressure Poisson solve (Solve, src/sim/solver.inl:356-379) on sm_100a.
 //
-// One cooperative, persistent kernel runs the whole solve for every scene of the handle:
-// FLUID cells are split into fixed-size chunks that belong to exactly one scene; each chunk
-// writes its partial dot products; the last block to arrive at a grid barrier reduces each
-// scene's chunk partials in a fixed order and updates that scene's alpha/beta/stop state.
-// Results therefore do not depend on block scheduling, nor on which other scenes share the
-// launch (a scene's chunk boundaries depend only on its own FLUID count).
+// Cooperative, persistent kernels run the whole solve for every scene of the handle.  FLUID cells
+// are split into chunks that belong to exactly one scene; each chunk writes its partial dot
+// products, and each scene's partials are reduced in a fixed order.  Results therefore do not
+// depend on block scheduling, nor on which other scenes share the launch (a scene's chunk
+// boundaries depend only on its own FLUID count).
+//   k_pcg_res (pcg_resident.cuh) -- FP64 and MIXED scenes whose state the SMs hold;
+//   k_pcg_fast -- the others, and REF32: state streamed through L2, one grid barrier an iteration;
+//   k_pcg -- launches with an ordered preconditioner: the last block to arrive at a grid barrier
+//            reduces the partials and updates every scene's alpha/beta/stop state.
 //
 // Precision modes:
 //   kRef32 -- the reference's fp32 arithmetic: ComputeAx's exact expression (solver.inl:196-230),

@@ -606,7 +606,7 @@ def main():
     # FLUID cells of all scenes from the per-scene sweep totals (cell_outer = sum nf * sweeps)
     fluid_cells = tot.cell_outer * b.k / max(tot.outer, 1)
     in_l2 = fluid_cells * (2 * 4 + 2) * (8 if args.precision == "fp64" else 4) < 100e6
-    roofline = {"kernel": "k_pcg_fast<%s> (persistent pressure solve)" % args.precision, "bound": "hbm",
+    roofline = {"kernel": "k_pcg_res / k_pcg_fast<%s> (persistent pressure solve)" % args.precision, "bound": "hbm",
                 "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": (achieved / peak) if achieved else None, "peak_source": peak_kind,
                 "traffic": traffic,
