@@ -297,7 +297,7 @@ __device__ __forceinline__ void write_pairs(const DevState& S, const SceneDev& D
     const uint32_t a = S.start[c], r = (uint32_t)s - a;
     if (r & 1u) return;
     if (s + 1 >= S.start[c + 1])
-        q = make_float4(kFar, kFar, kFar, 0.0f);
+        q = make_float4(p.x, p.y, p.z, 0.0f);
     else if ((threadIdx.x & 31) == 31)
         q = next_pos(s + 1);
     float4* const rec = S.spair + 2 * (size_t)(S.pstart[c] + r / 2);
@@ -357,8 +357,9 @@ __global__ void k_make_pairs(DevState S) {
 // candidates -- and reads the candidates two at a time as the records k_sort_permute pairs up:
 // a quarter of the records per pair of particles, and their terms as packed fp32x2 operations,
 // one candidate per lane of the pair.  Each particle's sum still adds its candidates one by one in
-// slot order, with the bits of the scalar expressions; the far second particle of an odd pair
-// adds +0.  128^3 dam break 0.645 -> 0.53 ms, 64^3 0.100 -> 0.082, 77^3 (no power of two) 0.248 ->
+// slot order, with the bits of the scalar expressions; the second particle of an odd pair, of mass 0
+// at the place of the first, adds +0 whatever the radius (a far one does not: with a squared radius
+// that overflows, its distance over the radius is no number).  128^3 dam break 0.645 -> 0.53 ms, 64^3 0.100 -> 0.082, 77^3 (no power of two) 0.248 ->
 // 0.168, with 0.03 ms (128^3) more in the sort; now bound by the fp32 pipe, 12 operations a
 // candidate.  Four or three blocks per SM measure the same, five 2-10% slower; unrolled by 4 2%
 // slower, not at all 4%.

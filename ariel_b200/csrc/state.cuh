@@ -31,7 +31,7 @@ struct DevState {
     float4* gpos4;    // slot -> P2G record: clamped grid position and mass (FLUID), far away
                       // for other particles so that they fall outside every face's radius
     // the slots' positions and masses as pairs inside a cell, for the density's packed arithmetic:
-    // (x0 x1 y0 y1), (z0 z1 m0 m1); the second of a cell's odd last particle is far away, mass 0
+    // (x0 x1 y0 y1), (z0 z1 m0 m1); the second of a cell's odd last particle is the same point, mass 0
     uint32_t* pstart;  // cell -> first pair (nc+1)
     float4* spair;
     float* dens;      // slot -> density

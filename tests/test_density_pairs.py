@@ -37,6 +37,29 @@ def test_density_bits(n, count, density):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("density", [1e25, 1e19, 1e-25])
+@pytest.mark.parametrize("count", [1, 2, 301])
+def test_density_bits_where_the_squared_radius_leaves_the_range(count, density):
+    """A kernel radius whose square overflows (every particle near counts with its whole mass) or
+    is zero (no number): cells of odd counts, whose last pair record is filled up."""
+    from oracle.pyoracle import RefSim
+    rng = np.random.default_rng(count)
+    desc = A.scene_dambreak(4, density=density)
+    pos = rng.random((count, 3)).astype(np.float32)
+    got = []
+    for make in (lambda: Batch([desc], params()), lambda: RefSim(desc, params())):
+        s = make()
+        s.set_particles(pos, np.zeros_like(pos), np.ones(count, np.float32), np.full(count, A.FLUID, np.int32))
+        s.stage(A.STAGE_SORT)
+        s.stage(A.STAGE_DENSITY)
+        got.append(s.get_particles()["density"])
+        s.close()
+    if density > 1:
+        assert not np.isnan(got[1]).any()
+    assert_bits("density", got[0], got[1])
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("graph", [0, 1])
 def test_density_after_the_resamplers_sort(graph):
     # no resampling: the step's last sort leaves every particle where a fresh sort finds it
