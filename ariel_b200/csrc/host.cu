@@ -718,26 +718,25 @@ ariel_status build_state(ariel_sim* s, std::vector<HostParticles>& hp, const ari
     A.S = S;
     s->pcg_blocks = pcg_max_blocks(s->device, s->mode, s->prm.pcg_blocks_per_sm);
     if (s->prm.pcg_grid_blocks > 0) s->pcg_blocks = std::min(s->pcg_blocks, (int)s->prm.pcg_grid_blocks);
-    A.res_blocks = pcg_res_blocks(s->device, s->mode);
+    A.classes = 0;
+    if (A.fast)
+        for (int i = 0; i < k; ++i) {
+            const long long n = s->descs[i].dim;
+            A.classes |= res_class_mask(s->mode, k, n * n * n);
+        }
+    A.res_blocks = pcg_res_blocks(s->device, s->mode, A.classes);
     if (s->prm.pcg_grid_blocks > 0) A.res_blocks = std::min(A.res_blocks, (int)s->prm.pcg_grid_blocks);
     A.all_resident = A.res_blocks > 0;
-    A.classes = 0;
-    for (int i = 0; i < k; ++i) {
+    for (int i = 0; i < k && A.all_resident; ++i) {
         // over the FLUID counts that the scene's grid allows: one per chunk size, and the largest
         const long long n = s->descs[i].dim, most = n * n * n;
+        const int m = (int)std::min(chunk_bound(most), kChunkTarget);
         for (int c = kChunkMin; c <= chunk_size(most); c += kChunkAlign) {
-            const int m = (int)std::min(chunk_bound(most), kChunkTarget);
-            A.classes |= 1 << res_class(k, c, m);
             const int cpb = res_max_cpb(s->mode, k, c, m);
             if (m > A.res_blocks * cpb || !res_never_over(s->mode, c, cpb)) A.all_resident = 0;
         }
-        if (chunk_bound(most) > kChunkTarget) {
-            A.classes |= 1 << kResBig;
-            A.all_resident = 0;
-        }
+        if (chunk_bound(most) > kChunkTarget) A.all_resident = 0;
     }
-    if (s->mode != kMixed) A.classes &= ~(1 << kResBig);
-    if (s->mode == kFp64 && k > 1) A.classes = A.all_resident = 0;
     cudaStream_t st = s->stream;
     // scene table and prefixes
     ARIEL_CUDA(cudaMemcpyAsync(s->d_scenes, s->sh.data(), sizeof(SceneDev) * k, cudaMemcpyHostToDevice, st));

@@ -2358,8 +2358,10 @@ template <int MODE>
 static cudaError_t launch_res(const PcgArgs& A, cudaStream_t st) {
     cudaError_t e = cudaSuccess;
     if (e == cudaSuccess && (A.classes & 1)) e = coop_launch_res<MODE, 0>(A, st);
-    if (e == cudaSuccess && (A.classes & 2)) e = coop_launch_res<MODE, 1>(A, st);
-    if (e == cudaSuccess && (A.classes & 4)) e = coop_launch_res<MODE, 2>(A, st);
+    if constexpr (MODE == kMixed) {
+        if (e == cudaSuccess && (A.classes & 2)) e = coop_launch_res<MODE, 1>(A, st);
+        if (e == cudaSuccess && (A.classes & 4)) e = coop_launch_res<MODE, 2>(A, st);
+    }
     if (e == cudaSuccess && (A.classes & 8)) e = coop_launch_res<MODE, 3>(A, st);
     if constexpr (MODE == kMixed)
         if (e == cudaSuccess && (A.classes & 16)) e = coop_launch_res<MODE, kResBig>(A, st);
@@ -2422,8 +2424,8 @@ int pcg_max_blocks(int device, int mode, int per_sm_cap) {
     return sms * (per < cap ? per : cap);
 }
 
-int pcg_res_blocks(int device, int mode) {
-    if (mode == kRef32) return 0;
+int pcg_res_blocks(int device, int mode, int classes) {
+    if (classes == 0) return 0;
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     auto fits = [](const void* f) {
@@ -2431,13 +2433,15 @@ int pcg_res_blocks(int device, int mode) {
         return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmem) == cudaSuccess &&
                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, kResThreads, kResSmem) == cudaSuccess && per > 0;
     };
-    const void* const f64[] = {(const void*)k_pcg_res<kFp64, 0>, (const void*)k_pcg_res<kFp64, 1>,
-                               (const void*)k_pcg_res<kFp64, 2>, (const void*)k_pcg_res<kFp64, 3>};
-    const void* const f32[] = {(const void*)k_pcg_res<kMixed, 0>, (const void*)k_pcg_res<kMixed, 1>,
-                               (const void*)k_pcg_res<kMixed, 2>, (const void*)k_pcg_res<kMixed, 3>,
-                               (const void*)k_pcg_res<kMixed, kResBig>};
+    // FP64 scenes are resident only alone, which leaves classes 0 and 3
+    const void* const f64[kResClasses] = {(const void*)k_pcg_res<kFp64, 0>, nullptr, nullptr,
+                                          (const void*)k_pcg_res<kFp64, 3>, nullptr};
+    const void* const f32[kResClasses] = {(const void*)k_pcg_res<kMixed, 0>, (const void*)k_pcg_res<kMixed, 1>,
+                                          (const void*)k_pcg_res<kMixed, 2>, (const void*)k_pcg_res<kMixed, 3>,
+                                          (const void*)k_pcg_res<kMixed, kResBig>};
     bool ok = true;
-    for (int c = 0; c < (mode == kFp64 ? 4 : 5); ++c) ok = ok && fits(mode == kFp64 ? f64[c] : f32[c]);
+    for (int c = 0; c < kResClasses; ++c)
+        if (classes >> c & 1) ok = ok && fits(mode == kFp64 ? f64[c] : f32[c]);
     if (!ok) cudaGetLastError();
     return ok ? sms : 0;  // 0: no scene is resident
 }

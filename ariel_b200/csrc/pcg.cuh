@@ -81,7 +81,7 @@ struct PcgArgs {
     unsigned* res_count;
     int res_blocks;            // its blocks (one per SM)
     int all_resident;          // every scene fits the resident solve whatever its FLUID cells are
-    int classes;               // bit c: some scene may be of class c
+    int classes;               // bit c: some scene may be of class c (res_class_mask)
     // per-cell operator data (dense over packed cells)
     uint8_t* mask;   // bit d set: neighbour d (-x,+x,-y,+y,-z,+z) is FLUID
     double* diag;    // ADiag (fp32 value for REF32, fp64 otherwise)
@@ -122,7 +122,7 @@ cudaError_t launch_pcg_prepare(const PcgArgs& A, uint32_t* pred, uint32_t* scan,
 cudaError_t launch_pcg_solve(const PcgArgs& A, int nblocks, cudaStream_t st);
 // Blocks of the persistent kernel that fit on the device at once; the resident solve's.
 int pcg_max_blocks(int device, int mode, int per_sm_cap);
-int pcg_res_blocks(int device, int mode);
+int pcg_res_blocks(int device, int mode, int classes);
 // Bounded-wait self test (one arrival missing).
 cudaError_t launch_barrier_selftest(Barrier* bar, int* err, unsigned long long timeout_ns, cudaStream_t st);
 
@@ -195,6 +195,18 @@ __host__ __device__ constexpr int res_max_cpb(int mode, int scenes, int csize, i
     int c = 2 * res_chunks(cls);
     while (c > 0 && !res_fits(mode, c * csize, cls == kResBig)) c >>= 1;
     return c;
+}
+// The classes (bit c: class c) that a scene on a grid of `cells` cells may be of, over the FLUID
+// counts that the grid allows: what a handle loads and launches.  A kernel that no scene of the
+// handle can reach is not looked at, since the first look loads it (a process's first handle, MIXED:
+// 32^3 6.7 -> 5.8 ms, 64^3 12.5 -> 11.9).  FP64 scenes are resident only alone (pcg_tables).
+inline int res_class_mask(int mode, int scenes, long long cells) {
+    if (mode == kRef32 || (mode == kFp64 && scenes > 1)) return 0;
+    const int chunks = (int)std::min(chunk_bound(cells), kChunkTarget);
+    int mask = mode == kMixed && chunk_bound(cells) > kChunkTarget ? 1 << kResBig : 0;
+    for (int c = kChunkMin; c <= chunk_size(cells); c += kChunkAlign)
+        if (res_max_cpb(mode, scenes, c, chunks) > 0) mask |= 1 << res_class(scenes, c, chunks);
+    return mask;
 }
 constexpr int kBrickMaxCells = 2048;
 constexpr int kBrickMaxExt = 2744;
