@@ -191,13 +191,26 @@ int mode_of(const AsimParams& p) {
     return p.precision == ARIEL_PREC_FP64 ? kFp64 : (p.precision == ARIEL_PREC_MIXED ? kMixed : kRef32);
 }
 
+constexpr long long round256(long long b) { return (b + 255) / 256 * 256; }
+
+// The pressure solve's vectors, one allocation: eight of a value per cell, then the packed ones of
+// four, four and two, each from a multiple of 256 bytes on.  `at`: where vector i begins.
+long long solver_vectors(int mode, long long nc, long long* at = nullptr) {
+    const long long vb = mode == kFp64 ? 8 : 4;
+    long long total = 0;
+    for (int i = 0; i < 11; ++i) {
+        if (at) at[i] = total;
+        total += round256((i < 8 ? 1 : (i < 10 ? 4 : 2)) * vb * std::max(1ll, nc));
+    }
+    return total;
+}
+
 // The allocation list of build_state, in bytes (each buffer rounded to 256 bytes as the
 // allocators place them).  Kept next to build_state; a GPU test holds the two equal.
 long long layout_bytes(const Layout& L) {
     long long total = 0;
     auto add = [&](long long count, long long esize) {
-        long long b = std::max(1ll, count) * esize;
-        total += (b + 255) / 256 * 256;
+        total += round256(std::max(1ll, count) * esize);
     };
     const long long k = L.k, np = L.np, nc = L.nc, nf = L.nf;
     add(k, sizeof(SceneDev));
@@ -216,10 +229,7 @@ long long layout_bytes(const Layout& L) {
     add(np, 16);  // spos4
     add(np, 16);  // svel4
     add(np, 16);  // gpos4
-    add(nc + 1, 4);  // pstart
-    add(pair_bound(np, nc), 32);  // spair
     add(np, 4);   // dens
-    add(np, 4);   // dens by id
     add(6 * np, 4);  // host I/O staging
     add(nc + 1, 4);  // solid_start
     add(nc, 1);      // flags
@@ -247,9 +257,7 @@ long long layout_bytes(const Layout& L) {
     add(nc, 8);      // diag
     add(nc, 8);      // pc64
     add(nc, 4);      // pc32
-    const long long vb = L.mode == kFp64 ? 8 : 4;
-    for (int i = 0; i < 8; ++i) add(nc, vb);
-    for (int i = 0; i < 3; ++i) add((i < 2 ? 4 : 2) * nc, vb);
+    add(solver_vectors(L.mode, nc), 1);
     if (L.mode == kMixed) {
         add(nc, 8);
         add(nc, 4);
@@ -578,10 +586,7 @@ ariel_status build_state(ariel_sim* s, std::vector<HostParticles>& hp, const ari
     ARIEL_TRY(dalloc(s, &S.spos4, np));
     ARIEL_TRY(dalloc(s, &S.svel4, np));
     ARIEL_TRY(dalloc(s, &S.gpos4, np));
-    ARIEL_TRY(dalloc(s, &S.pstart, nc + 1));
-    ARIEL_TRY(dalloc(s, &S.spair, 2 * (size_t)pair_bound(np, nc)));
     ARIEL_TRY(dalloc(s, &S.dens, np));
-    ARIEL_TRY(dalloc(s, &s->d_dens_id, np));
     ARIEL_TRY(dalloc(s, &s->d_stage, 6 * (size_t)np));
     ARIEL_TRY(dalloc(s, &S.solid_start, nc + 1, true));
     ARIEL_TRY(dalloc(s, &S.flags, nc));
@@ -637,22 +642,27 @@ ariel_status build_state(ariel_sim* s, std::vector<HostParticles>& hp, const ari
     ARIEL_TRY(dalloc(s, &A.diag, nc));
     ARIEL_TRY(dalloc(s, &A.pc64, nc));
     ARIEL_TRY(dalloc(s, &A.pc32, nc));
-    const size_t vb = s->mode == kFp64 ? 8 : 4;
-    char* v[8];
-    for (int i = 0; i < 8; ++i) ARIEL_TRY(dalloc(s, &v[i], vb * (size_t)nc));
-    A.r = v[0];
-    A.z = v[1];
-    A.s0 = v[2];
-    A.s1 = v[3];
-    A.q = v[4];
-    A.ordq = v[5];
-    A.u = v[6];
-    A.p = v[7];
-    char* w4[3];
-    for (int i = 0; i < 3; ++i) ARIEL_TRY(dalloc(s, &w4[i], (i < 2 ? 4 : 2) * vb * (size_t)nc));
-    A.va0 = w4[0];
-    A.va1 = w4[1];
-    A.vb = w4[2];
+    long long at[11];
+    char* vec = nullptr;
+    ARIEL_TRY(dalloc(s, &vec, (size_t)solver_vectors(s->mode, nc, at)));
+    A.r = vec + at[0];
+    A.z = vec + at[1];
+    A.s0 = vec + at[2];
+    A.s1 = vec + at[3];
+    A.q = vec + at[4];
+    A.ordq = vec + at[5];
+    A.u = vec + at[6];
+    A.p = vec + at[7];
+    A.va0 = vec + at[8];
+    A.va1 = vec + at[9];
+    A.vb = vec + at[10];
+    // The density's pair records live from a sort to the density after it, when the I/O staging
+    // area, the solver's vectors and its scan are all free (pairs_stale: any of them has been used
+    // since, or the sort was the resampler's).  At most 16 (np + min(np, nc) + 1) bytes: from two
+    // particles a cell on they fit the staging area's 24 np; below, 48 nc + 48 bytes hold them, of the
+    // vectors' 72 nc or more.  As buffers of their own they took 0.7 GB for a 256^3 scene.
+    S.spair = 32 * pair_bound(np, nc) <= 24 * np ? (float4*)s->d_stage : (float4*)vec;
+    S.pstart = s->flscan;
     if (s->mode == kMixed) {
         ARIEL_TRY(dalloc(s, &A.r64, nc));
         ARIEL_TRY(dalloc(s, &A.d32, nc));
@@ -949,6 +959,7 @@ ariel_status enqueue_stage(ariel_sim* s, int g, cudaEvent_t* evs = nullptr) {
         case ARIEL_STAGE_CLASSIFY: e = launch_classify(S, 0, st); break;
         case ARIEL_STAGE_BOUNDARY_DIV: e = launch_boundary_div(S, st); break;
         case ARIEL_STAGE_SOLVE:
+            s->pairs_stale = true;
             e = launch_pcg_prepare(s->PA, s->flpred, s->flscan, s->scan_tmp, st);
             if (e == cudaSuccess && evs) e = cudaEventRecordWithFlags(evs[kEvSolveKernel], st, cudaEventRecordExternal);
             if (e == cudaSuccess) e = launch_pcg_solve(s->PA, s->pcg_blocks, st);
@@ -1337,9 +1348,10 @@ ariel_status ariel_get_particles(ariel_sim* s, int32_t scene, float* pos, float*
     ARIEL_CUDA(cudaStreamSynchronize(s->stream));
     const long long b = s->ppref[scene], n = s->ppref[scene + 1] - b;
     if (n == 0) return ARIEL_OK;
-    // two rounds through the I/O staging area: positions and velocities, then mass and type (and
-    // the densities from their own buffer)
+    // two rounds through the I/O staging area: positions and velocities, then mass, type and the
+    // densities (of all scenes, by id)
     float* const stage = s->d_stage;
+    s->pairs_stale = true;
     if (pos || vel) {
         ARIEL_CUDA(launch_pack_state(s->S.pos4 + b, s->S.vel4 + b, stage, stage + 3 * n, n, s->stream));
         std::vector<HostPiece> h;
@@ -1353,8 +1365,8 @@ ariel_status ariel_get_particles(ariel_sim* s, int32_t scene, float* pos, float*
         if (mass) h.push_back({mass, stage, 4 * (size_t)n});
         if (type) h.push_back({type, stage + n, 4 * (size_t)n});
         if (density) {
-            ARIEL_CUDA(launch_scatter_density(s->S, s->d_dens_id, s->stream));
-            h.push_back({density, s->d_dens_id + b, 4 * (size_t)n});
+            ARIEL_CUDA(launch_scatter_density(s->S, stage + 2 * n, s->stream));
+            h.push_back({density, stage + 2 * n + b, 4 * (size_t)n});
         }
         ARIEL_CUDA(download(s->stream, h));
     }
@@ -1527,6 +1539,7 @@ ariel_status ariel_upload_state(ariel_sim* s, int32_t scene, const float* pos, c
     if (n == 0) return ARIEL_OK;
     float* sp = s->d_stage;
     float* sv = s->d_stage + 3 * n;
+    s->pairs_stale = true;
     ARIEL_CUDA(cudaMemcpyAsync(sp, pos, 12 * (size_t)n, cudaMemcpyHostToDevice, s->stream));
     ARIEL_CUDA(cudaMemcpyAsync(sv, vel, 12 * (size_t)n, cudaMemcpyHostToDevice, s->stream));
     ARIEL_CUDA(launch_unpack_state(s->S.pos4 + b, s->S.vel4 + b, sp, sv, n, s->S.dev_error, s->stream));
@@ -1539,6 +1552,7 @@ ariel_status ariel_download_state(ariel_sim* s, int32_t scene, float* pos, float
     if (n > 0) {
         float* sp = s->d_stage;
         float* sv = s->d_stage + 3 * n;
+        s->pairs_stale = true;
         ARIEL_CUDA(launch_pack_state(s->S.pos4 + b, s->S.vel4 + b, sp, sv, n, s->stream));
         ARIEL_CUDA(cudaMemcpyAsync(pos, sp, 12 * (size_t)n, cudaMemcpyDeviceToHost, s->stream));
         ARIEL_CUDA(cudaMemcpyAsync(vel, sv, 12 * (size_t)n, cudaMemcpyDeviceToHost, s->stream));

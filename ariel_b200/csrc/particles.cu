@@ -335,7 +335,8 @@ __global__ void k_sort_permute(DevState S) {
     S.gpos4[s] = gp;
 }
 
-// The pair records of slots sorted without them (the resampler's Sort).
+// The pair records of slots that have been sorted: where the sort was the resampler's, which leaves them
+// out, or their memory has been used since.
 __global__ void k_make_pairs(DevState S) {
     kernel_begin();
     SCENE_PREFIX(S.p_pref);

@@ -91,7 +91,7 @@ struct ariel_sim {
     long long np = 0, nc = 0, nf = 0;
     bool any_solid = false;
     bool inited = false;
-    bool pairs_stale = false;  // the last sort queued was the resampler's
+    bool pairs_stale = false;  // the density's pair records are not there (build_state)
     cudaStream_t stream = nullptr;
     bool own_stream = true;
     cudaMemPool_t pool = nullptr;  // set: every buffer comes from this stream-ordered pool
@@ -103,7 +103,6 @@ struct ariel_sim {
     ariel::PcgArgs PA{};
     void* scan_tmp = nullptr;
     uint32_t *flpred = nullptr, *flscan = nullptr;
-    float* d_dens_id = nullptr;
     int pcg_blocks = 0;
     int mode = ariel::kRef32;
     // graphs of one whole step: [0] plain, [1],[2] with the two stage-event sets

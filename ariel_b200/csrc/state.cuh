@@ -60,7 +60,8 @@ struct DevState {
 // Launchers (each returns cudaGetLastError()).
 cudaError_t launch_begin(const DevState& S, cudaStream_t st);
 cudaError_t launch_sort(const DevState& S, void* scan_tmp, cudaStream_t st);
-// the density's pair records when the last sort was the resampler's, which leaves them out
+// the density's pair records where the last sort's are not there any more, or it was the resampler's,
+// which leaves them out
 cudaError_t launch_make_pairs(const DevState& S, void* scan_tmp, cudaStream_t st);
 cudaError_t launch_density(const DevState& S, cudaStream_t st);
 cudaError_t launch_forces(const DevState& S, cudaStream_t st);
