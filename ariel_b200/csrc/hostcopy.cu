@@ -6,6 +6,7 @@
 // them: 10 MB into fresh pages 4.55 -> 2.3 ms, 2.5 MB 1.16 -> 0.8 ms, 40 MB 18.2 -> 6.4 ms.
 // Nothing is allocated: pinned chunks of the framework's own reach the same rates, but pinning
 // 8 MB of them cost the first copy after a handle's creation 4 to 8 ms.
+#include <sched.h>
 #include <sys/mman.h>
 #include <unistd.h>
 
@@ -31,7 +32,15 @@ constexpr size_t kFresh = 1024 * 1024;
 // Ready bytes that the caller copies at a time while others still work (the copies wait for
 // the device one by one: 512 KB each reach 10.5 GB/s, 2.5 MB 15.8).
 constexpr size_t kRun = 2 * 1024 * 1024;
-constexpr int kWorkers = 4;  // host threads of one copy, the caller among them
+// Host threads of one copy, the caller among them: at most four, and no more than the CPUs that the
+// caller may run on, where more of them would only take turns with it.
+int workers() {
+    constexpr int kMost = 4;
+    cpu_set_t may;
+    if (sched_getaffinity(0, sizeof(may), &may) != 0)  // more CPUs than the set holds
+        return kMost;
+    return std::min(kMost, std::max(1, CPU_COUNT(&may)));
+}
 
 // Joins its threads when it goes.
 struct Helpers {
@@ -99,7 +108,7 @@ cudaError_t download_i32(cudaStream_t st, const HostPiece& h) {
         for (size_t i = next++; i < n; i = next++)
             for (size_t j = i * kElems, end = std::min(j + kElems, h.bytes); j < end; ++j) out[j] = f[j];
     };
-    Helpers helpers((int)std::min<size_t>(kWorkers, n) - 1, work);
+    Helpers helpers((int)std::min<size_t>(workers(), n) - 1, work);
     work();
     return cudaSuccess;
 }
@@ -136,7 +145,7 @@ cudaError_t download(cudaStream_t st, const std::vector<HostPiece>& pieces) {
             ready[i].store(true, std::memory_order_release);
             return true;
         };
-        Helpers helpers((int)std::min<size_t>(kWorkers, (n + 1) / 2) - 1, [&] {
+        Helpers helpers((int)std::min<size_t>(workers(), (n + 1) / 2) - 1, [&] {
             while (take()) {
             }
         });

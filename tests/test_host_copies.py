@@ -2,6 +2,8 @@
 is read back, around the sizes where the copy changes its form (the driver's staging alone below
 1 MB or into mapped pages, then behind threads that map the pages in parts of 512 KB), from several
 threads at once, and with the particles equal to those of the pinned-buffer path."""
+import os
+import subprocess
 import threading
 
 import numpy as np
@@ -78,3 +80,17 @@ def test_particles_equal_the_pinned_path(n):
         assert (q["mass"] == 1).all() and (q["type"] == A.FLUID).all()
         assert np.isfinite(q["density"]).all()
     b.close()
+
+
+@pytest.mark.gpu
+def test_host_threads_of_a_copy(tmp_path):
+    """tests/cpp/host_copies.cpp: as many threads as the caller may use CPUs, at most."""
+    from ariel_b200 import build as B
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    libdir = os.path.join(root, "ariel_b200", "_lib")
+    exe = str(tmp_path / "host_copies")
+    subprocess.run([B.host_compiler(), "-std=c++17", "-O1", "-I", os.path.join(root, "include"),
+                    os.path.join(root, "tests", "cpp", "host_copies.cpp"), "-L", libdir, "-lariel_b200",
+                    "-Wl,-rpath," + libdir, "-rdynamic", "-ldl", "-pthread", "-o", exe], check=True, capture_output=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout.strip() == "ok", (r.returncode, r.stdout, r.stderr)
