@@ -1354,21 +1354,23 @@ ariel_status ariel_get_particles(ariel_sim* s, int32_t scene, float* pos, float*
     s->pairs_stale = true;
     if (pos || vel) {
         ARIEL_CUDA(launch_pack_state(s->S.pos4 + b, s->S.vel4 + b, stage, stage + 3 * n, n, s->stream));
-        std::vector<HostPiece> h;
-        if (pos) h.push_back({pos, stage, 12 * (size_t)n});
-        if (vel) h.push_back({vel, stage + 3 * n, 12 * (size_t)n});
-        ARIEL_CUDA(download(s->stream, h));
+        HostPiece h[2];
+        int m = 0;
+        if (pos) h[m++] = {pos, stage, 12 * (size_t)n};
+        if (vel) h[m++] = {vel, stage + 3 * n, 12 * (size_t)n};
+        ARIEL_CUDA(download(s->stream, h, m));
     }
     if (density || mass || type) {
-        std::vector<HostPiece> h;
+        HostPiece h[3];
+        int m = 0;
         if (mass || type) ARIEL_CUDA(launch_pack_w(s->S.pos4 + b, s->S.vel4 + b, stage, (int32_t*)(stage + n), n, s->stream));
-        if (mass) h.push_back({mass, stage, 4 * (size_t)n});
-        if (type) h.push_back({type, stage + n, 4 * (size_t)n});
+        if (mass) h[m++] = {mass, stage, 4 * (size_t)n};
+        if (type) h[m++] = {type, stage + n, 4 * (size_t)n};
         if (density) {
             ARIEL_CUDA(launch_scatter_density(s->S, stage + 2 * n, s->stream));
-            h.push_back({density, stage + 2 * n + b, 4 * (size_t)n});
+            h[m++] = {density, stage + 2 * n + b, 4 * (size_t)n};
         }
-        ARIEL_CUDA(download(s->stream, h));
+        ARIEL_CUDA(download(s->stream, h, m));
     }
     return ARIEL_OK;
 }
@@ -1383,7 +1385,8 @@ ariel_status ariel_get_cells(ariel_sim* s, int32_t scene, int32_t* particle_cell
         ARIEL_CUDA(copy_sync(s->stream, key.data(), s->S.key + pb, pn * sizeof(uint32_t), cudaMemcpyDeviceToHost));
         for (long long i = 0; i < pn; ++i) particle_cell[i] = (int32_t)((long long)key[i] - cb);
     }
-    if (cell_count) ARIEL_CUDA(download(s->stream, {{cell_count, s->S.count + cb, cn * sizeof(uint32_t)}}));
+    const HostPiece counts{cell_count, s->S.count + cb, cn * sizeof(uint32_t)};
+    if (cell_count) ARIEL_CUDA(download(s->stream, &counts, 1));
     return ARIEL_OK;
 }
 
@@ -1417,7 +1420,8 @@ ariel_status ariel_get_grid(ariel_sim* s, int32_t scene, int32_t which, void* bu
     ARIEL_TRY(grid_span(s, scene, which, &d, &elems, &esize, &flags));
     if ((size_t)nbytes != elems * esize) return ARIEL_ERR_INVALID_ARG;
     ARIEL_CUDA(cudaStreamSynchronize(s->stream));
-    ARIEL_CUDA(download(s->stream, {{buf, d, flags ? elems : elems * esize, flags}}));
+    const HostPiece h{buf, d, flags ? elems : elems * esize, flags};
+    ARIEL_CUDA(download(s->stream, &h, 1));
     return ARIEL_OK;
 }
 

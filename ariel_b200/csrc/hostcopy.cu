@@ -13,9 +13,9 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdint>
+#include <exception>
 #include <memory>
 #include <new>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -48,13 +48,11 @@ struct Helpers {
     // up to `n` threads (fewer if they cannot be started) that run `work`
     template <class F>
     Helpers(int n, const F& work) {
-        t.reserve((size_t)std::max(n, 0));
-        for (int i = 0; i < n; ++i) {
-            try {
-                t.emplace_back(work);
-            } catch (const std::system_error&) {
-                break;
-            }
+        try {
+            t.reserve((size_t)std::max(n, 0));
+            for (int i = 0; i < n; ++i) t.emplace_back(work);
+        } catch (const std::exception&) {
+            // no memory or no thread: those that there are do the work, the caller at least
         }
     }
     ~Helpers() {
@@ -98,7 +96,8 @@ void touch(char* p, size_t bytes, size_t page) {
 cudaError_t download_i32(cudaStream_t st, const HostPiece& h) {
     const std::unique_ptr<uint8_t[]> f(new (std::nothrow) uint8_t[h.bytes]);
     if (!f) return cudaErrorMemoryAllocation;
-    cudaError_t e = download(st, {{f.get(), h.dev, h.bytes}});
+    const HostPiece bytes{f.get(), h.dev, h.bytes};
+    cudaError_t e = download(st, &bytes, 1);
     if (e != cudaSuccess) return e;
     int32_t* const out = static_cast<int32_t*>(h.host);
     constexpr size_t kElems = kPart / sizeof(int32_t);
@@ -115,26 +114,33 @@ cudaError_t download_i32(cudaStream_t st, const HostPiece& h) {
 
 }  // namespace
 
-cudaError_t download(cudaStream_t st, const std::vector<HostPiece>& pieces) {
+// Throws nothing: without memory for its lists every piece goes the driver's way alone.
+cudaError_t download(cudaStream_t st, const HostPiece* pieces, int count) {
     struct Part {
         const HostPiece* h;
         size_t off, bytes;
     };
     const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-    std::vector<Part> parts;
     size_t total = 0;
-    for (const HostPiece& h : pieces)
-        if (!h.to_i32) total += h.bytes;
-    std::vector<const HostPiece*> plain;
-    for (const HostPiece& h : pieces) {
-        if (h.bytes == 0 || h.to_i32) continue;
-        if (total >= kFresh && fresh(static_cast<const char*>(h.host), h.bytes, page))
-            for (size_t o = 0; o < h.bytes; o += kPart) parts.push_back({&h, o, std::min(kPart, h.bytes - o)});
-        else
-            plain.push_back(&h);
+    for (int i = 0; i < count; ++i)
+        if (!pieces[i].to_i32) total += pieces[i].bytes;
+    std::vector<Part> parts;
+    std::vector<std::atomic<bool>> ready;
+    auto in_parts = [&](const HostPiece& h) {
+        return std::any_of(parts.begin(), parts.end(), [&](const Part& p) { return p.h == &h; });
+    };
+    try {
+        for (int i = 0; i < count; ++i) {
+            const HostPiece& h = pieces[i];
+            if (h.bytes == 0 || h.to_i32) continue;
+            if (total >= kFresh && fresh(static_cast<const char*>(h.host), h.bytes, page))
+                for (size_t o = 0; o < h.bytes; o += kPart) parts.push_back({&h, o, std::min(kPart, h.bytes - o)});
+        }
+        ready = std::vector<std::atomic<bool>>(parts.size());
+    } catch (const std::bad_alloc&) {
+        parts.clear();
     }
     const size_t n = parts.size();
-    std::vector<std::atomic<bool>> ready(n);
     std::atomic<size_t> next{0};
     cudaError_t e = cudaSuccess;
     {
@@ -169,11 +175,15 @@ cudaError_t download(cudaStream_t st, const std::vector<HostPiece>& pieces) {
         };
         while (take()) flush(false);
         flush(true);
-        for (const HostPiece* h : plain)
-            if (e == cudaSuccess) e = cudaMemcpyAsync(h->host, h->dev, h->bytes, cudaMemcpyDeviceToHost, st);
     }
-    for (const HostPiece& h : pieces)
-        if (h.to_i32 && h.bytes && e == cudaSuccess) e = download_i32(st, h);
+    for (int i = 0; i < count && e == cudaSuccess; ++i) {
+        const HostPiece& h = pieces[i];
+        if (h.bytes == 0) continue;
+        if (h.to_i32)
+            e = download_i32(st, h);
+        else if (!in_parts(h))
+            e = cudaMemcpyAsync(h.host, h.dev, h.bytes, cudaMemcpyDeviceToHost, st);
+    }
     const cudaError_t se = cudaStreamSynchronize(st);
     return e != cudaSuccess ? e : se;
 }

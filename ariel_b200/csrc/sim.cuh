@@ -140,7 +140,7 @@ struct HostPiece {
     size_t bytes;  // on the device
     bool to_i32 = false;
 };
-cudaError_t download(cudaStream_t st, const std::vector<HostPiece>& pieces);
+cudaError_t download(cudaStream_t st, const HostPiece* pieces, int count);
 
 ariel_status validate(const AsimSceneDesc& d);
 SceneDev make_scene(const AsimSceneDesc& d, const AsimParams& p);

@@ -224,7 +224,8 @@ ariel_status ariel_get_level_set(ariel_sim* s, int32_t scene, float* phi, int64_
     float* d_phi = nullptr;
     cudaError_t e = T.alloc(&d_phi, m);
     if (e == cudaSuccess) e = level_set(s, scene, d_phi, N);
-    if (e == cudaSuccess) e = download(s->stream, {{phi, d_phi, m * sizeof(float)}});
+    const HostPiece out{phi, d_phi, m * sizeof(float)};
+    if (e == cudaSuccess) e = download(s->stream, &out, 1);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return map_cuda_error(e, "ariel_get_level_set");
@@ -272,10 +273,11 @@ ariel_status ariel_surface_mesh(ariel_sim* s, int32_t scene, float* vertices, in
         count_launch(4);
         e = cudaGetLastError();
     }
-    std::vector<HostPiece> out;
-    if (vertices && (int64_t)nv <= max_vertices) out.push_back({vertices, d_v, (size_t)nv * sizeof(float3)});
-    if (quads && (int64_t)nq <= max_quads) out.push_back({quads, d_q, (size_t)nq * sizeof(int4)});
-    if (e == cudaSuccess) e = download(st, out);
+    HostPiece out[2];
+    int pieces = 0;
+    if (vertices && (int64_t)nv <= max_vertices) out[pieces++] = {vertices, d_v, (size_t)nv * sizeof(float3)};
+    if (quads && (int64_t)nq <= max_quads) out[pieces++] = {quads, d_q, (size_t)nq * sizeof(int4)};
+    if (e == cudaSuccess) e = download(st, out, pieces);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return map_cuda_error(e, "ariel_surface_mesh");

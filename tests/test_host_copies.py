@@ -82,15 +82,25 @@ def test_particles_equal_the_pinned_path(n):
     b.close()
 
 
-@pytest.mark.gpu
-def test_host_threads_of_a_copy(tmp_path):
-    """tests/cpp/host_copies.cpp: as many threads as the caller may use CPUs, at most."""
+def _run_cpp(tmp_path, name):
     from ariel_b200 import build as B
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     libdir = os.path.join(root, "ariel_b200", "_lib")
-    exe = str(tmp_path / "host_copies")
+    exe = str(tmp_path / name)
     subprocess.run([B.host_compiler(), "-std=c++17", "-O1", "-I", os.path.join(root, "include"),
-                    os.path.join(root, "tests", "cpp", "host_copies.cpp"), "-L", libdir, "-lariel_b200",
+                    os.path.join(root, "tests", "cpp", name + ".cpp"), "-L", libdir, "-lariel_b200",
                     "-Wl,-rpath," + libdir, "-rdynamic", "-ldl", "-pthread", "-o", exe], check=True, capture_output=True)
     r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout.strip() == "ok", (r.returncode, r.stdout, r.stderr)
+
+
+@pytest.mark.gpu
+def test_host_threads_of_a_copy(tmp_path):
+    """tests/cpp/host_copies.cpp: as many threads as the caller may use CPUs, at most."""
+    _run_cpp(tmp_path, "host_copies")
+
+
+@pytest.mark.gpu
+def test_copies_without_host_memory(tmp_path):
+    """tests/cpp/host_copy_memory.cpp: a failed allocation in a copy is a status, or no matter."""
+    _run_cpp(tmp_path, "host_copy_memory")
