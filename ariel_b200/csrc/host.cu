@@ -760,6 +760,7 @@ ariel_status build_state(ariel_sim* s, std::vector<HostParticles>& hp, const ari
     ARIEL_CUDA(cudaMemsetAsync(S.pu, 0, sizeof(float) * nf, st));
     ARIEL_CUDA(cudaMemsetAsync(S.flags, 0, nc, st));
     ARIEL_CUDA(cudaMemsetAsync(A.sc, 0, sizeof(PcgScene) * k, st));
+    ARIEL_CUDA(cudaMemsetAsync(A.res, 0xff, sizeof(int4) * k, st));  // no scene resident
     if (!bricks.empty())
         ARIEL_CUDA(copy_sync(st, dbr, bricks.data(), bricks.size() * sizeof(int4), cudaMemcpyHostToDevice));
     ARIEL_CUDA(copy_sync(st, dbase, bbase.data(), bbase.size() * sizeof(int), cudaMemcpyHostToDevice));
@@ -1587,6 +1588,14 @@ ariel_status ariel_selftest_barrier_timeout(double timeout_ms) {
     cudaFree(err);
     if (e != cudaSuccess) return map_cuda_error(e);
     return h ? ARIEL_ERR_DEVICE_TIMEOUT : ARIEL_OK;
+}
+
+ariel_status ariel_selftest_solve_resident(ariel_sim* s, int32_t scene, int32_t* resident) {
+    if (!s || !resident || scene < 0 || scene >= s->k) return ARIEL_ERR_INVALID_ARG;
+    int4 place{};
+    ARIEL_CUDA(copy_sync(s->stream, &place, s->PA.res + scene, sizeof(place), cudaMemcpyDeviceToHost));
+    *resident = place.x >= 0;
+    return ARIEL_OK;
 }
 
 // ---- checkpoints -------------------------------------------------------------------------

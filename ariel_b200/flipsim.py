@@ -203,6 +203,12 @@ class Batch:
         check(self.L.ariel_solver_totals(self.h, scene, C.byref(t)), "ariel_solver_totals")
         return t
 
+    def solve_resident(self, scene=0):
+        """Whether the scene's last pressure solve ran in the resident kernel (tests, tuning)."""
+        r = C.c_int32()
+        check(self.L.ariel_selftest_solve_resident(self.h, scene, C.byref(r)), "ariel_selftest_solve_resident")
+        return bool(r.value)
+
     def timer_begin(self):
         check(self.L.ariel_timer_begin(self.h), "ariel_timer_begin")
 

@@ -276,6 +276,9 @@ ariel_status ariel_timing_get(ariel_sim* sim, double* ms, double* solve_kernel_m
  * that it must time out after `timeout_ms`; returns ARIEL_ERR_DEVICE_TIMEOUT when the bound
  * worked and ARIEL_OK if the barrier (wrongly) completed. */
 ariel_status ariel_selftest_barrier_timeout(double timeout_ms);
+/* Which kernel the scene's last pressure solve ran in (tests and tuning; results do not depend on
+ * it): *resident 1 for the one that keeps a scene on the SMs, 0 for the others, 0 before a solve. */
+ariel_status ariel_selftest_solve_resident(ariel_sim* sim, int32_t scene, int32_t* resident);
 
 /* Static solid meshes: the reference's solid mesh geoms (Scene's solids built from OBJ files,
  * src/scene/scene.cpp:362-434, src/geom/obj/obj.cpp) for scenes that reference them through

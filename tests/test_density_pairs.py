@@ -73,3 +73,24 @@ def test_density_after_the_resamplers_sort(graph):
     for s in range(2):
         assert_bits("scene %d" % s, b.get_particles(s)["density"], stale[s])
     b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [13, 20])
+def test_density_after_a_resampling_that_moved_particles(n):
+    """The resampler sorts the advected particles and then moves them; the records made after it are
+    those of its sort, so the density is that of a sort and a density in the resampler's place."""
+    got = []
+    for stages in ((A.STAGE_SORT, A.STAGE_DENSITY), (A.STAGE_RESAMPLE, A.STAGE_DENSITY)):
+        b = Batch([dambreak(n), dambreak(n - 4, seed=3)], params())
+        b.init()
+        b.step(2)
+        for g in range(A.STAGE_RESAMPLE):
+            b.stage(g)
+        for g in stages:
+            b.stage(g)
+        got.append([b.get_particles(s) for s in range(2)])
+        b.close()
+    for s in range(2):
+        assert (got[0][s]["pos"] != got[1][s]["pos"]).any()
+        assert_bits("scene %d" % s, got[1][s]["density"], got[0][s]["density"])
