@@ -672,7 +672,7 @@ ariel_status build_state(ariel_sim* s, std::vector<HostParticles>& hp, const ari
     ARIEL_TRY(dalloc(s, &A.res, k));
     ARIEL_TRY(dalloc(s, &A.res_count, 32 * (size_t)k));
     A.flscan = s->flscan;
-    A.hlist = s->flpred;  // free once the list is written
+    A.hlist = (uint32_t*)A.z;  // z to p, which only REF32 and the ordered solves use: 7 nc words in MIXED
     // bricks of the ordered sweeps: every scene's brick grid, listed by level I+J+K, then scene
     // and position (the order the sweeps take them in)
     sweep_brick(s->prm, A.bx, A.by, A.bz);

@@ -72,7 +72,7 @@ struct PcgArgs {
     uint4* rec;                // per FLUID-list entry: (cell, neighbour mask, diagonal bits)
     const long long* fl_pref;  // k+1
     const long long* ch_pref;  // k+1 chunk begins (scenes of the resident solve have none)
-    uint32_t* hlist;           // resident solve, largest class: the blocks' halo positions
+    uint32_t* hlist;           // resident solve, largest class: halo positions, 6 per FLUID-list entry
     const uint32_t* flscan;    // packed cell in list_order -> FLUID-list position
     // resident solve: per scene (first block position, positions, chunks, first partial), or
     // position kNotResident; one arrival counter per scene, 128 bytes apart, with a word that a

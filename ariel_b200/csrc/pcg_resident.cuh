@@ -84,15 +84,16 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
     // Shared memory: per cell (p, x), the diagonal, pc, u and three words of neighbour positions in
     // u (x, y, z pairs of 14 bits; bit 28 of the first: some neighbour lies in another block); u
     // continues with the halo -- the neighbours in other blocks -- and a slot that stays 0 for
-    // neighbours that are not FLUID; the halo's list positions, where its owners publish.
-    const int cells = cpb * csize, hslots = res_halo_slots(MODE, cells, BIG);
-    const int hcap = BIG ? min(hslots, blen) : hslots, zero = cells + hcap;
+    // neighbours that are not FLUID; the halo's list positions, where its owners publish.  BIG: these in
+    // hlist, which has six for every list position (a slot a cell was too few for a scene's last block,
+    // often a short one: its neighbours are mostly not its own, and the scene was handed over).
+    const int cells = cpb * csize, hcap = res_halo_slots(MODE, cells, BIG), zero = cells + hcap;
     T2* const px = BIG ? (T2*)A.vb + t0 : reinterpret_cast<T2*>(dyn);
     T* const dgs = reinterpret_cast<T*>(dyn + (BIG ? 0 : sizeof(T2) * cells));
     T* const pcs = dgs + cells;
     T* const ub = pcs + cells;
     uint32_t* const nw = reinterpret_cast<uint32_t*>(ub + zero + 1);
-    uint32_t* const hpos = BIG ? A.hlist + t0 : nw + 3 * cells;
+    uint32_t* const hpos = BIG ? A.hlist + 6 * t0 : nw + 3 * cells;
     const uint32_t* const cs = A.fl + t0;
     const unsigned arrivals = (unsigned)pl.y;
     unsigned* const count = A.res_count + 32 * (size_t)sc;
@@ -418,8 +419,13 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
                 const int h = tid + u * kResThreads;
                 if (h < nhalo) ub[cells + h] = u_of(eh[u]);
             }
+            // (BIG: hpos made anew from t0, which is at hand: kept across the iterations, its registers
+            // are spilled elsewhere, 160^3 6.0 -> 6.4 ms)
+            long long tb = t0;
+            if (BIG) asm volatile("" : "+l"(tb));
+            const uint32_t* const hp = BIG ? A.hlist + 6 * tb : hpos;
             for (int h = tid + kAhead * kResThreads; h < nhalo; h += kResThreads)
-                ub[cells + h] = u_of(ldcg4(Ac + hpos[h]));
+                ub[cells + h] = u_of(ldcg4(Ac + hp[h]));
             T2 bc[BIG ? kGroup : 1];
 #pragma unroll
             for (int q = 0; q < R; ++q) {

@@ -102,6 +102,18 @@ def test_neighbours_without_room(precision, scene):
     _assert_same(got[0], want[0])
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("last", [1, 33, 700, 2048, 3001, 4095, 4096, 4097, 6000, 8191])
+def test_big_scene_with_a_short_last_block(last):
+    # 74 blocks of four full chunks and one of `last` cells, whose neighbours are mostly not its own
+    scene = _first(90, 296 * 2048 + last)
+    got, where = _solve([scene], A.PREC_MIXED)
+    assert where == [True]
+    want, where = _solve([scene], A.PREC_MIXED, 24)
+    assert where == [False]
+    _assert_same(got[0], want[0])
+
+
 MIX = {
     "shared": lambda: _first(58, 296 * 640),      # chunks of 640 cells, four to a block
     "pair": lambda: _first(69, 296 * 1100),       # two to a block, all blocks
