@@ -1575,19 +1575,19 @@ ariel_status ariel_selftest_barrier_timeout(double timeout_ms) {
     Barrier* bar = nullptr;
     int* err = nullptr;
     ARIEL_CUDA(cudaMalloc(&bar, sizeof(Barrier)));
-    if (cudaMalloc(&err, sizeof(int)) != cudaSuccess) {
+    int h[3] = {};
+    if (cudaMalloc(&err, sizeof(h)) != cudaSuccess) {
         cudaFree(bar);
         return ARIEL_ERR_OOM;
     }
-    cudaMemset(err, 0, sizeof(int));
+    cudaMemset(err, 0, sizeof(h));
     cudaError_t e = launch_barrier_selftest(bar, err, (unsigned long long)(timeout_ms * 1.0e6), 0);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    int h = 0;
-    if (e == cudaSuccess) e = copy_sync(0, &h, err, sizeof(int), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = copy_sync(0, h, err, sizeof(h), cudaMemcpyDeviceToHost);
     cudaFree(bar);
     cudaFree(err);
     if (e != cudaSuccess) return map_cuda_error(e);
-    return h ? ARIEL_ERR_DEVICE_TIMEOUT : ARIEL_OK;
+    return h[0] && h[1] ? ARIEL_ERR_DEVICE_TIMEOUT : ARIEL_OK;
 }
 
 ariel_status ariel_selftest_solve_resident(ariel_sim* s, int32_t scene, int32_t* resident) {

@@ -2449,7 +2449,8 @@ int pcg_res_blocks(int device, int mode, int classes) {
 cudaError_t launch_barrier_selftest(Barrier* bar, int* err, unsigned long long timeout_ns, cudaStream_t st) {
     cudaMemsetAsync(bar, 0, sizeof(Barrier), st);
     k_barrier_selftest<<<2, 32, 0, st>>>(bar, err, timeout_ns);
-    count_launch();
+    k_wait_selftest<<<1, 64, 0, st>>>(bar, reinterpret_cast<unsigned*>(err) + 2, err + 1, timeout_ns);
+    count_launch(2);
     return cudaGetLastError();
 }
 

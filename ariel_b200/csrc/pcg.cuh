@@ -123,7 +123,8 @@ cudaError_t launch_pcg_solve(const PcgArgs& A, int nblocks, cudaStream_t st);
 // Blocks of the persistent kernel that fit on the device at once; the resident solve's.
 int pcg_max_blocks(int device, int mode, int per_sm_cap);
 int pcg_res_blocks(int device, int mode, int classes);
-// Bounded-wait self test (one arrival missing).
+// Self tests of the bounded waits (one arrival missing): err[0] for the grid barrier's, err[1] for the
+// resident solve's, 1 where it gave up as it should; err[2] is theirs.
 cudaError_t launch_barrier_selftest(Barrier* bar, int* err, unsigned long long timeout_ns, cudaStream_t st);
 
 constexpr int kPcgThreads = 256;

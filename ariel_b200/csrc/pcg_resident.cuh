@@ -33,6 +33,60 @@ __device__ __forceinline__ double4 ldcg4(const double4* p) {
     return make_double4(a.x, a.y, b.x, b.y);
 }
 
+// Waits until `want` arrivals are counted.  Bounded: gives up, with the error words set, when nothing has
+// moved for `timeout_ns`, or when another block has given up.  The beat counts the exchanges of all
+// scenes, since a block of the scene that is waited for may still be busy with one of an earlier group.
+__device__ __forceinline__ bool wait_arrivals(const unsigned* count, unsigned want, Barrier* bar, int* dev_error,
+                                              unsigned long long timeout_ns) {
+    unsigned spin = 0, beat = 0;
+    unsigned long long t_start = 0;
+    while (ld_acquire_cnt(count) < want) {
+        if ((++spin & 255u) != 0) continue;
+        if (*(volatile int*)&bar->error) return false;
+        const unsigned long long now = gtimer();
+        const unsigned bt = *(volatile unsigned*)&bar->beat;
+        if (t_start == 0 || bt != beat) {
+            t_start = now;
+            beat = bt;
+        } else if (now - t_start > timeout_ns) {
+            atomicExch(&bar->error, 1);
+            if (dev_error) atomicExch(dev_error, 1);
+            return false;
+        }
+    }
+    return true;
+}
+
+// Self test of that wait, one block: an arrival that never comes, one that comes after three times
+// the limit while others move, and an error of another block.  1 into *err when it did as it
+// should.
+__global__ void k_wait_selftest(Barrier* bar, unsigned* count, int* err, unsigned long long timeout_ns) {
+    const int tid = threadIdx.x;
+    if (tid == 0) {
+        *bar = Barrier{};
+        *count = 0;
+        const bool gave_up = !wait_arrivals(count, 1u, bar, nullptr, timeout_ns) && *(volatile int*)&bar->error == 1;
+        *err = gave_up;
+        *bar = Barrier{};
+        __threadfence();
+    }
+    __syncthreads();
+    if (tid == 32) {
+        for (int i = 0; i < 6; ++i) {
+            const unsigned long long t0 = gtimer();
+            while (gtimer() - t0 < timeout_ns / 2) __nanosleep(1000);
+            atomicAdd(&bar->beat, 1u);
+        }
+        red_release_add(count, 1u);
+    } else if (tid == 0) {
+        const bool came = wait_arrivals(count, 1u, bar, nullptr, timeout_ns) && *(volatile int*)&bar->error == 0;
+        atomicExch(&bar->error, 1);
+        const unsigned long long t0 = gtimer();
+        const bool left = !wait_arrivals(count, 2u, bar, nullptr, timeout_ns) && gtimer() - t0 < timeout_ns;
+        *err = *err && came && left;
+    }
+}
+
 // One block per SM: two halves of kPcgThreads threads, each with one chunk or more.  Fewer arrivals and
 // pollers make the barrier cheaper than two blocks per SM do (148 against 291 blocks: 2.2 against
 // 2.9 us for an arrival, the wait and the reading of three sums per chunk).
@@ -143,30 +197,7 @@ __device__ __forceinline__ bool res_scene(const PcgArgs& A, int sc, int v) {
             // release: orders the block's writes (collected by the barrier above) before the
             // arrival; acquire: the others' writes before what follows the barrier below
             red_release_add(count, 1u);
-            const unsigned want = epoch * arrivals;
-            unsigned spin = 0, beat = 0;
-            unsigned long long t_start = 0;
-            while (ld_acquire_cnt(count) < want) {
-                if ((++spin & 255u) != 0) continue;
-                // Bounded: gives up when nothing has moved for the time limit.  The beat
-                // counts the exchanges of all scenes, since a block of this scene may still
-                // be busy with a scene of an earlier group.
-                if (*(volatile int*)&A.bar->error) {
-                    ok = false;
-                    break;
-                }
-                const unsigned long long now = gtimer();
-                const unsigned bt = *(volatile unsigned*)&A.bar->beat;
-                if (t_start == 0 || bt != beat) {
-                    t_start = now;
-                    beat = bt;
-                } else if (now - t_start > tmo) {
-                    atomicExch(&A.bar->error, 1);
-                    if (S.dev_error) atomicExch(S.dev_error, 1);
-                    ok = false;
-                    break;
-                }
-            }
+            ok = wait_arrivals(count, epoch * arrivals, A.bar, S.dev_error, tmo);
             if (ch0 == 0) atomicAdd(&A.bar->beat, 1u);
         }
         return __syncthreads_and(ok) != 0;

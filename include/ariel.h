@@ -156,7 +156,9 @@ typedef struct AsimParams {
                                  replaces rand() (particleresampler.inl:69-71) */
     int32_t use_graph;        /* capture one step per CUDA graph and replay it */
     int32_t timing;           /* record per-stage CUDA-event times (adds event records) */
-    double barrier_timeout_ms;/* bound of every device-side spin wait */
+    double barrier_timeout_ms;/* bound of every device-side spin wait: how long it may last or, in the
+                                 solve of scenes that stay on the SMs, how long without an exchange of
+                                 any of them completed */
     int32_t fail_on_not_converged; /* return ARIEL_ERR_NOT_CONVERGED from step when a solve
                                       stops at max_iters above tolerance */
     int32_t pcg_blocks_per_sm;  /* blocks per SM of the persistent solve kernel; 0 = default (2) */
@@ -272,9 +274,10 @@ ariel_status ariel_solver_totals(ariel_sim* sim, int32_t scene, AsimSolverTotals
 ariel_status ariel_timing_get(ariel_sim* sim, double* ms, double* solve_kernel_ms, double* step_ms,
                               int32_t max_steps, int32_t* nsteps);
 
-/* Device-side failure detection: runs the bounded grid barrier with one arrival missing so
- * that it must time out after `timeout_ms`; returns ARIEL_ERR_DEVICE_TIMEOUT when the bound
- * worked and ARIEL_OK if the barrier (wrongly) completed. */
+/* Device-side failure detection: runs the bounded grid barrier, and the wait of the solve that keeps
+ * scenes on the SMs, with one arrival missing so that they must time out after `timeout_ms` (the
+ * latter also with arrivals that come late, while others move); returns ARIEL_ERR_DEVICE_TIMEOUT when
+ * the bounds worked and ARIEL_OK if a wait (wrongly) completed. */
 ariel_status ariel_selftest_barrier_timeout(double timeout_ms);
 /* Which kernel the scene's last pressure solve ran in (tests and tuning; results do not depend on
  * it): *resident 1 for the one that keeps a scene on the SMs, 0 for the others, 0 before a solve. */
