@@ -1463,7 +1463,7 @@ __device__ bool count_barrier(Barrier* bar, int* dev_error, unsigned epoch, unsi
         red_release_add(&bar->count, 1u);
         const unsigned target = epoch * gridDim.x;
         const unsigned long long t0 = gtimer();
-        while (ld_acquire_cnt(&bar->count) < target) {
+        while (!arrived(ld_acquire_cnt(&bar->count), target)) {
             if (*(volatile int*)&bar->error) {
                 s_ok = 0;
                 break;

@@ -151,6 +151,11 @@ inline long long chunk_bound(long long cells) {
     const long long hi = (cells + kChunkMax - 1) / kChunkMax;
     return std::min(lo, std::max(kChunkTarget, hi));
 }
+// Whether a counter of arrivals has come to `want`.  Both wrap around in a solve of more than 2^32 arrivals
+// (a tolerance out of reach, n^3 iterations: from 310^3 on); they are never 2^31 apart.
+__host__ __device__ constexpr bool arrived(unsigned count, unsigned want) { return count - want < 0x80000000u; }
+static_assert(arrived(5u, 5u) && arrived(6u, 5u) && !arrived(4u, 5u), "plain counts");
+static_assert(arrived(3u, 0xfffffff0u) && !arrived(0xfffffff0u, 3u), "counts on both sides of 2^32");
 // The resident solve: scenes of one chunk or more per block (one block per SM) whose cells fit its
 // shared memory together with slots for neighbours in other blocks.
 constexpr int kResMaxChunks = 320;   // what the reduction of a scene's partials reads in one go:

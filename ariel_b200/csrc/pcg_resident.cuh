@@ -40,7 +40,7 @@ __device__ __forceinline__ bool wait_arrivals(const unsigned* count, unsigned wa
                                               unsigned long long timeout_ns) {
     unsigned spin = 0, beat = 0;
     unsigned long long t_start = 0;
-    while (ld_acquire_cnt(count) < want) {
+    while (!arrived(ld_acquire_cnt(count), want)) {
         if ((++spin & 255u) != 0) continue;
         if (*(volatile int*)&bar->error) return false;
         const unsigned long long now = gtimer();
@@ -58,13 +58,13 @@ __device__ __forceinline__ bool wait_arrivals(const unsigned* count, unsigned wa
 }
 
 // Self test of that wait, one block: an arrival that never comes, one that comes after three times
-// the limit while others move, and an error of another block.  1 into *err when it did as it
-// should.
+// the limit while others move, and an error of another block, with the count wrapping around at the
+// first two arrivals.  1 into *err when it did as it should.
 __global__ void k_wait_selftest(Barrier* bar, unsigned* count, int* err, unsigned long long timeout_ns) {
     const int tid = threadIdx.x;
     if (tid == 0) {
         *bar = Barrier{};
-        *count = 0;
+        *count = 0xffffffffu;
         const bool gave_up = !wait_arrivals(count, 1u, bar, nullptr, timeout_ns) && *(volatile int*)&bar->error == 1;
         *err = gave_up;
         *bar = Barrier{};
@@ -77,7 +77,7 @@ __global__ void k_wait_selftest(Barrier* bar, unsigned* count, int* err, unsigne
             while (gtimer() - t0 < timeout_ns / 2) __nanosleep(1000);
             atomicAdd(&bar->beat, 1u);
         }
-        red_release_add(count, 1u);
+        red_release_add(count, 2u);
     } else if (tid == 0) {
         const bool came = wait_arrivals(count, 1u, bar, nullptr, timeout_ns) && *(volatile int*)&bar->error == 0;
         atomicExch(&bar->error, 1);
