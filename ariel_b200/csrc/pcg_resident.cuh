@@ -59,9 +59,12 @@ __device__ __forceinline__ bool wait_arrivals(const unsigned* count, unsigned wa
 
 // Self test of that wait, one block: an arrival that never comes, one that comes after three times
 // the limit while others move, and an error of another block, with the count wrapping around at the
-// first two arrivals.  1 into *err when it did as it should.
+// first two arrivals.  1 into *err when it did as it should.  The latter two with a limit of at most 50 ms,
+// so that the test of a long one takes little longer than the limit; the last has 5 ms more than half the
+// limit, since the wait looks at the error every 256 polls.
 __global__ void k_wait_selftest(Barrier* bar, unsigned* count, int* err, unsigned long long timeout_ns) {
     const int tid = threadIdx.x;
+    const unsigned long long limit = timeout_ns < 50000000ull ? timeout_ns : 50000000ull;
     if (tid == 0) {
         *bar = Barrier{};
         *count = 0xffffffffu;
@@ -74,15 +77,15 @@ __global__ void k_wait_selftest(Barrier* bar, unsigned* count, int* err, unsigne
     if (tid == 32) {
         for (int i = 0; i < 6; ++i) {
             const unsigned long long t0 = gtimer();
-            while (gtimer() - t0 < timeout_ns / 2) __nanosleep(1000);
+            while (gtimer() - t0 < limit / 2) __nanosleep(1000);
             atomicAdd(&bar->beat, 1u);
         }
         red_release_add(count, 2u);
     } else if (tid == 0) {
-        const bool came = wait_arrivals(count, 1u, bar, nullptr, timeout_ns) && *(volatile int*)&bar->error == 0;
+        const bool came = wait_arrivals(count, 1u, bar, nullptr, limit) && *(volatile int*)&bar->error == 0;
         atomicExch(&bar->error, 1);
         const unsigned long long t0 = gtimer();
-        const bool left = !wait_arrivals(count, 2u, bar, nullptr, timeout_ns) && gtimer() - t0 < timeout_ns;
+        const bool left = !wait_arrivals(count, 2u, bar, nullptr, limit) && gtimer() - t0 < limit / 2 + 5000000ull;
         *err = *err && came && left;
     }
 }

@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 from ariel_b200 import _abi as A
+from ariel_b200._lib import lib
 from ariel_b200.flipsim import Batch
 
 from helpers import dambreak, params
@@ -168,3 +169,9 @@ def test_steps_streamed(descs, blocks, graph):
             assert counts == counts0
             for key in ("pos", "vel"):
                 np.testing.assert_array_equal(p[key].view(np.uint8), q[key].view(np.uint8))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("timeout_ms", [0.0, 0.05, 1.0, 200.0])
+def test_bounded_waits_at_any_limit(timeout_ms):
+    assert lib().ariel_selftest_barrier_timeout(timeout_ms) == A.ARIEL_ERR_DEVICE_TIMEOUT
