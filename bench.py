@@ -602,11 +602,29 @@ def main():
     else:
         workload_key = "pcg_%s_%s%d" % (args.precision, args.workload, args.n)
     traffic = load_traffic(workload_key)
-    # the solve's packed state (Av twice, Bv) of the FLUID cells fits the 126 MB L2 or not;
-    # FLUID cells of all scenes from the per-scene sweep totals (cell_outer = sum nf * sweeps)
+    # Where the solve's state lies: on the SMs for the whole solve (k_pcg_res), or packed in L2 or HBM
+    # (k_pcg_fast: Av twice and Bv of the FLUID cells, in the 126 MB L2 or not); FLUID cells of all
+    # scenes from the per-scene sweep totals (cell_outer = sum nf * sweeps)
+    resident = [b.solve_resident(i) for i in range(b.k)]
+    solvers = (["k_pcg_res"] if any(resident) else []) + (["k_pcg_fast"] if not all(resident) else [])
     fluid_cells = tot.cell_outer * b.k / max(tot.outer, 1)
     in_l2 = fluid_cells * (2 * 4 + 2) * (8 if args.precision == "fp64" else 4) < 100e6
-    roofline = {"kernel": "k_pcg_res / k_pcg_fast<%s> (persistent pressure solve)" % args.precision, "bound": "hbm",
+    if all(resident):
+        limit = ("the exchange between blocks in every iteration (arrival, wait, partial sums, scalar divisions) and "
+                 "the neighbour gather in shared memory, not bandwidth")
+        note = ("nominal, not bandwidth use: the fixed bytes a cell over the time. The iteration state stays in registers and "
+                "shared memory; only cells with a neighbour in another block and the partial sums cross L2 (a committed "
+                "capture of the 128^3 dam break: 26 MB of DRAM traffic a solve, 15.7 MB of L2 traffic an iteration)")
+    else:
+        limit = "load latency at 16 warps per SM"
+        note = ("the streamed scenes' working set stays in L2 at this size, so DRAM traffic is far below the algorithmic bytes"
+                if in_l2 else "the solve's working set exceeds L2: DRAM traffic includes the streamed 16-byte cell "
+                "records (about 16 B per FLUID cell per iteration)")
+        if any(resident):
+            limit += "; scenes that fit the SMs: the exchange between blocks in every iteration"
+            note += "; %d of %d scenes are resident on the SMs" % (sum(resident), len(resident))
+    roofline = {"kernel": "%s<%s> (persistent pressure solve)" % (" / ".join(solvers), args.precision), "bound": "hbm",
+                "limited_by": limit,
                 "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": (achieved / peak) if achieved else None, "peak_source": peak_kind,
                 "traffic": traffic,
@@ -621,11 +639,7 @@ def main():
                 "own_model": "%g B per cell-iteration: the single-reduction algorithm's own traffic"
                              % PCG_BYTES_PER_CELL_ITER[key],
                 "avg_launch_ms": solve_ms,
-                "note": "frac of %s HBM copy bandwidth; " % peak_kind +
-                        ("the solve's working set stays in L2 at this size, so DRAM traffic is far below "
-                         "the algorithmic bytes" if in_l2 else
-                         "the solve's working set exceeds L2: DRAM traffic includes the streamed "
-                         "16-byte cell records (about 16 B per FLUID cell per iteration)")}
+                "note": "frac of %s HBM copy bandwidth; %s" % (peak_kind, note)}
 
     # every stage against HBM with its per-particle and per-cell bytes, from the same CUDA-event
     # stage times (stages with several kernels are timed as one)
