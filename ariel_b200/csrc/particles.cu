@@ -353,7 +353,7 @@ __global__ void k_make_pairs(DevState S) {
 //
 // The kernel radius is 2 cells, so nearly all of the 27 cells' 216 particles count.  One particle
 // per thread reading one 16-byte record per candidate was bound by what L1 returns to the
-// registers (86% of its wavefronts; a warp's 16-byte loads take four however many lanes share
+// registers (85% of its wavefronts; a warp's 16-byte loads take four however many lanes share
 // an address).  Here a thread takes the two particles of a pair -- the same cell, so the same
 // candidates -- and reads the candidates two at a time as the records k_sort_permute pairs up:
 // a quarter of the records per pair of particles, and their terms as packed fp32x2 operations,
@@ -361,8 +361,8 @@ __global__ void k_make_pairs(DevState S) {
 // slot order, with the bits of the scalar expressions; the second particle of an odd pair, of mass 0
 // at the place of the first, adds +0 whatever the radius (a far one does not: with a squared radius
 // that overflows, its distance over the radius is no number).  128^3 dam break 0.645 -> 0.53 ms, 64^3 0.100 -> 0.082, 77^3 (no power of two) 0.248 ->
-// 0.168, with 0.03 ms (128^3) more in the sort; now bound by the fp32 pipe, 12 operations a
-// candidate.  Four or three blocks per SM measure the same, five 2-10% slower; unrolled by 4 2%
+// 0.168, with 0.03 ms (128^3) more in the sort.  A third fewer instructions; L1's wavefronts at 82% of
+// their peak (85% before) and the fp32 pipe at 74% (52%), 12 operations a candidate, bind it now.  Four or three blocks per SM measure the same, five 2-10% slower; unrolled by 4 2%
 // slower, not at all 4%.
 // ------------------------------------------------------------------------------------------
 __device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
@@ -383,8 +383,9 @@ __device__ __forceinline__ float min_nan(float x, float y) {
 // quotient estimate r2 * inv, inv the rounded 1 / hh, is corrected by its exact remainder, which
 // gives the correctly rounded quotient (Markstein, IBM J. Res. Dev. 34, 1990) -- checked against
 // the division for every r2 up to 8 hh at 40 grid sizes.  r2 is held to 8 hh (weight 0, as beyond
-// it) so that the remainder of an infinite one is no NaN; a remainder that underflows changes
-// quotients below 2^-70, which 1 - q does not see.
+// it) so that the remainder of an infinite one is no NaN; a remainder is a multiple of 2^-46 times the
+// product of hh's and q's leading bits, so for hh above 2^-60 only those of quotients below 2^-42
+// can underflow, which 1 - q does not see.
 // kDivPlain (radii out of any scene's range): the division.
 // The assembler contracts a packed multiply that feeds a packed add into one rounding, whatever
 // --fmad says, so such products are fused adds of `nzero`, a -0 that it cannot see through.

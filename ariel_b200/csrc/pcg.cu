@@ -175,8 +175,9 @@ struct VT<kFp64> {
 // compact piece of the liquid, with about 0.6 neighbours outside it per cell where a chunk of whole
 // grid rows has 2.1, and still runs of up to 32 consecutive cells along z (resident solve at
 // 128^3: 2.70 -> 2.21 ms).  FP64 keeps the grid's order, whose chunks of the list its dot products
-// follow: they are the only thing that the order enters, in the last bit, and fp64 scalars carry
-// it into the pressure where the fp32 modes round it off.
+// follow: they are the only thing that the order enters, in the last bits, and fp64 scalars carry
+// it into the pressure.  The fp32 modes round alpha and beta to 24 bits and so lose it nearly always
+// (a last bit that moves a scalar across an fp32 rounding moves the pressure's last bits).
 __device__ __forceinline__ int list_order(int mode, int n, int i, int j, int k) {
     if (mode == kFp64) return (i * n + j) * n + k;
     const int i0 = i & ~7, j0 = j & ~7, k0 = k & ~31;

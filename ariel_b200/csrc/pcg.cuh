@@ -152,7 +152,7 @@ inline long long chunk_bound(long long cells) {
     return std::min(lo, std::max(kChunkTarget, hi));
 }
 // Whether a counter of arrivals has come to `want`.  Both wrap around in a solve of more than 2^32 arrivals
-// (a tolerance out of reach, n^3 iterations: from 310^3 on); they are never 2^31 apart.
+// (a tolerance out of reach, n^3 iterations, 296 blocks: from 245^3 on); they are never 2^31 apart.
 __host__ __device__ constexpr bool arrived(unsigned count, unsigned want) { return count - want < 0x80000000u; }
 static_assert(arrived(5u, 5u) && arrived(6u, 5u) && !arrived(4u, 5u), "plain counts");
 static_assert(arrived(3u, 0xfffffff0u) && !arrived(0xfffffff0u, 3u), "counts on both sides of 2^32");

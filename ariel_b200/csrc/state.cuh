@@ -100,7 +100,7 @@ void count_launch(int n = 1);
 long long launch_count();
 
 // Launch with programmatic stream serialisation; `k` must begin with kernel_begin().  The launch
-// latency of a kernel is then hidden behind its predecessor: a step is about 35 launches (44 before the
+// latency of a kernel is then hidden behind its predecessor: a step is 37 launches at 128^3 (nine more before the
 // clears, the scan of the tile sums and the solver tables were folded into other kernels), most of
 // them of a few microseconds on small grids.  Step, ms: 32^3 0.699 -> 0.643, 64^3 1.402 -> 1.368.
 template <class... P, class... A>
